@@ -1,0 +1,602 @@
+// Run-time compiled passes: the source generator.
+//
+// A register pass planned by build_reg can also run as a kernel generated for
+// it alone: every op, slot mask, control and relayout address is a constant
+// of the generated code, so there is no per-op dispatch, plain exchanges
+// (X, CX, SWAP without outside controls) become register renamings, zero and
+// unit matrix entries drop out of the arithmetic, and the matrices are read
+// as constant-bank operands from the launch's parameter block.  The source
+// depends on the pass's structure and on which matrix entries are exactly
+// 0, 1 or -1, not on the other matrix values, so passes of the same shape
+// share one compiled kernel (jit.cu caches by source text).
+#include <algorithm>
+#include <array>
+#include <cstdarg>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "common.cuh"
+#include "passgen.h"
+#include "regtile.cuh"
+
+namespace qs {
+
+bool jit_single_buffer(bool c128) {
+    static const int env = [] {
+        const char* e = getenv("QS_JIT_SINGLE_BUFFER");
+        return e && (*e == '0' || *e == '1') ? *e - '0' : -1;
+    }();
+    return env >= 0 ? env == 1 : c128;
+}
+
+namespace {
+
+constexpr size_t kJitMaxParamBytes = 32000;  // below the 32764-byte kernel parameter limit
+
+struct SrcBuf {
+    std::string s;
+    bool truncated = false;  // a formatted piece did not fit: the source is not used
+    void add(const char* fmt, ...) __attribute__((format(printf, 2, 3))) {
+        char tmp[1024];
+        va_list ap;
+        va_start(ap, fmt);
+        int k = vsnprintf(tmp, sizeof(tmp), fmt, ap);
+        va_end(ap);
+        if (k >= int(sizeof(tmp))) {
+            truncated = true;
+            k = int(sizeof(tmp)) - 1;
+        }
+        s.append(tmp, size_t(k));
+    }
+};
+
+// XOR of per-thread-bit images over the set bits of threadIdx.x, as an expression
+std::string thread_xor_expr(const uint32_t* img, int nT) {
+    std::string e;
+    for (int i = 0; i < nT; ++i) {
+        if (!img[i]) continue;
+        char t[64];
+        snprintf(t, sizeof(t), "%s(((tid >> %d) & 1u) * %uu)", e.empty() ? "" : " ^ ", i, img[i]);
+        e += t;
+    }
+    return e.empty() ? std::string("0u") : e;
+}
+
+// devfn != nullptr: emit the pass as `extern "C" __device__ void <devfn>(vec,
+// params, mats, partials, tile, tend, zero_in)` for the persistent batch
+// kernel instead of a kernel: it runs tiles [tile, tend) of the calling CTA,
+// reads its parameter block from global memory (params), may run in a CTA
+// wider than its own thread count (the other threads share the loads, repeat
+// the register work of thread tid mod threads, and store nothing), and with
+// zero_in != 0 reads |0...0> instead of the vector.
+template <typename V>
+bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_source = true,
+                  const char* devfn = nullptr) {
+    constexpr bool C128 = sizeof(V) == 16;
+    const int E = 1 << R, nT = a.nT, K = a.K, L = a.L, H = a.H;
+    const int threads = 1 << nT, nwarps = threads / 32;
+    const int NM = a.nmats > 0 ? a.nmats : 1;
+    const int NOPS = a.nops > 0 ? a.nops : 1;
+    const int NEXP = a.nexp > 0 ? a.nexp : 1;
+    const bool batched = a.batched != 0;
+    // ---- parameter block (all fields 8-byte aligned, V first):
+    //   V m[NM]; u64 ntiles, gthr[8], gslot[E], hibit[16], gctrl[NOPS], hsh[4 NOPS],
+    //   mgoff[NOPS], mstride[NOPS], eslot[NEXP], misc[2]; u32 pe[NM]
+    // m holds every op's matrix in slot order; for a batched pass the ops with
+    // per-instance tables (stride != 0) are staged into shared memory per
+    // instance instead: pe[g] = (op << 16) | offset within the instance block
+    const size_t o_ntiles = sizeof(V) * size_t(NM), o_gthr = o_ntiles + 8, o_gslot = o_gthr + 64,
+                 o_hibit = o_gslot + 8 * size_t(E), o_gctrl = o_hibit + 128, o_hsh = o_gctrl + 8 * size_t(NOPS),
+                 o_mgoff = o_hsh + 32 * size_t(NOPS), o_mstride = o_mgoff + 8 * size_t(NOPS),
+                 o_eslot = o_mstride + 8 * size_t(NOPS), o_misc = o_eslot + 8 * size_t(NEXP), o_pe = o_misc + 16;
+    size_t bytes = o_pe + (batched ? 4 * size_t(NM) : 0);
+    bytes = (bytes + 15) & ~size_t(15);
+    if (bytes > kJitMaxParamBytes) return false;
+    out.params.assign(bytes / 8, 0);
+    unsigned char* pb = reinterpret_cast<unsigned char*>(out.params.data());
+    auto put64 = [&](size_t off, uint64_t v) { memcpy(pb + off, &v, 8); };
+    V* pm = reinterpret_cast<V*>(pb);
+    std::vector<char> strided(size_t(NOPS), 0);
+    for (int o = 0; o < a.nops; ++o) {
+        const KCopy& c = a.cp[o];
+        const int D = 1 << c.m;
+        const int cnt = c.diag ? D : D * D;
+        strided[o] = batched && c.stride != 0;
+        put64(o_mgoff + 8 * size_t(o), uint64_t(c.goff));
+        put64(o_mstride + 8 * size_t(o), uint64_t(c.stride));
+        for (int e = 0; e < cnt; ++e) {
+            const int kr = c.diag ? e : e / D, kc = c.diag ? 0 : e % D;
+            int sr = 0, sc = 0;
+            for (int i = 0; i < c.m; ++i) {
+                sr |= ((kr >> i) & 1) << c.perm[i];
+                sc |= ((kc >> i) & 1) << c.perm[i];
+            }
+            const int src = c.diag ? sr : sr * D + sc;
+            if (strided[o]) {  // bit 31 marks a staged entry
+                const uint32_t v = (1u << 31) | (uint32_t(o) << 16) | uint32_t(src);
+                memcpy(pb + o_pe + 4 * size_t(c.soff + e), &v, 4);
+            } else {
+                pm[c.soff + e] = hm[c.goff + src];
+            }
+        }
+    }
+    if (a.nops > 32767) return false;
+    // tile position of the psi/lam pair bit (adjoint pair passes)
+    int pair_tile = -1;
+    for (int b = 0; b < 64 && a.pairmask; ++b)
+        if ((a.pairmask >> b) & 1) {
+            if (b < L) pair_tile = b;
+            for (int t = 0; t < H; ++t)
+                if (a.hi[t] == b) pair_tile = L + t;
+        }
+    auto gbit = [&](int b) -> uint64_t { return uint64_t(1) << (b < L ? b : a.hi[b - L]); };
+    const KStage& SL = a.st[a.nstages - 1];
+    put64(o_ntiles, uint64_t(1) << (a.n - K));
+    for (int i = 0; i < nT; ++i) put64(o_gthr + 8 * i, gbit(SL.T[i]));
+    for (int s = 0; s < E; ++s) {
+        uint64_t v = 0;
+        for (int j = 0; j < R; ++j)
+            if ((s >> j) & 1) v |= gbit(SL.R[j]);
+        put64(o_gslot + 8 * s, v);
+    }
+    for (int t = 0; t < H; ++t) put64(o_hibit + 8 * t, uint64_t(1) << a.hi[t]);
+    for (int o = 0; o < a.nops; ++o) {
+        put64(o_gctrl + 8 * o, a.ops[o].gctrl);
+        for (int q = 0; q < a.ops[o].nh; ++q)
+            put64(o_hsh + 32 * o + 8 * q, a.ops[o].hsrc[q] >= 64 ? uint64_t(a.ops[o].hsrc[q] - 64) : 0);
+    }
+    for (int e = 0; e < a.nexp; ++e) put64(o_eslot + 8 * e, uint64_t(a.eslot[e]));
+    put64(o_misc, ~a.pairmask);
+    put64(o_misc + 8, uint64_t(a.inst_shift));
+    // value class of a matrix entry: 0, 1, -1, general (3), real (4), imaginary
+    // (5).  An entry of a per-instance table gets the class that holds for
+    // every instance's value (e.g. real for the entries of Ry tables, imaginary
+    // for the off-diagonal entries of Rx tables); the value itself is read from
+    // the staged table at run time.
+    auto value_class = [](const V v) -> int {
+        if (v.y == 0) {
+            if (v.x == 0) return 0;
+            if (v.x == 1) return 1;
+            if (v.x == -1) return 2;
+            return 4;
+        }
+        return v.x == 0 ? 5 : 3;
+    };
+    auto join_class = [](int c1, int c2) -> int {
+        if (c1 == c2) return c1;
+        const bool r1 = c1 == 0 || c1 == 1 || c1 == 2 || c1 == 4, r2 = c2 == 0 || c2 == 1 || c2 == 2 || c2 == 4;
+        if (r1 && r2) return 4;
+        if ((c1 == 0 || c1 == 5) && (c2 == 0 || c2 == 5)) return 5;
+        return 3;
+    };
+    // instances of a batched pass: the vector bits above inst_shift, less the pair bit
+    const int64_t ninst =
+        batched && a.inst_shift > 0 ? (int64_t(1) << (a.n - a.inst_shift - (a.pairmask ? 1 : 0))) : int64_t(1);
+    std::vector<uint8_t> scls(size_t(NM), 3);
+    for (int o = 0; o < a.nops; ++o) {
+        if (!strided[o]) continue;
+        const KCopy& c = a.cp[o];
+        const int D = 1 << c.m;
+        const int cnt = c.diag ? D : D * D;
+        for (int e = 0; e < cnt; ++e) {
+            const int kr = c.diag ? e : e / D, kc = c.diag ? 0 : e % D;
+            int sr = 0, sc = 0;
+            for (int i = 0; i < c.m; ++i) {
+                sr |= ((kr >> i) & 1) << c.perm[i];
+                sc |= ((kc >> i) & 1) << c.perm[i];
+            }
+            const int64_t src = c.goff + (c.diag ? sr : sr * D + sc);
+            int cl = value_class(hm[src]);
+            for (int64_t i = 1; i < ninst && cl != 3; ++i) cl = join_class(cl, value_class(hm[src + i * c.stride]));
+            scls[size_t(c.soff + e)] = uint8_t(cl);
+        }
+    }
+    auto vclass = [&](int o, int idx) -> int { return strided[o] ? int(scls[size_t(idx)]) : value_class(pm[idx]); };
+    auto mref = [&](int o, int idx) -> std::string {
+        return (strided[o] ? "msm[" : "p.m[") + std::to_string(idx) + "]";
+    };
+    out.classes.resize(size_t(NM));
+    for (int o = 0; o < a.nops; ++o) {
+        const KCopy& c = a.cp[o];
+        const int cnt = c.diag ? (1 << c.m) : (1 << (2 * c.m));
+        for (int e = 0; e < cnt; ++e) out.classes[c.soff + e] = uint8_t(vclass(o, c.soff + e));
+    }
+    // Diagonal tables indexed by thread bits (a different entry per lane) are
+    // copied to shared memory once per CTA: parameter-space loads with lane-
+    // dependent addresses are serialised, shared-memory loads are not.
+    std::vector<int> doff(size_t(NOPS), -1);
+    int ndsm = 0;
+    for (int o = 0; o < a.nops; ++o) {
+        const KOp& op = a.ops[o];
+        const bool dg = op.code == QS_OP_DIAG || (op.code == QS_OP_EXPECT && (op.flags & QS_OPF_DIAG));
+        if (!dg || op.nh == 0 || strided[o]) continue;
+        bool thr = false;
+        for (int q = 0; q < op.nh; ++q) thr = thr || op.hsrc[q] < 64;
+        if (!thr) continue;
+        doff[size_t(o)] = ndsm;
+        ndsm += 1 << a.cp[o].m;
+    }
+    // the table of a diagonal with other-bit index h, as an expression prefix
+    auto dtab = [&](int o) -> std::string {
+        if (strided[o]) return "msm[" + std::to_string(int(a.ops[o].moff)) + " + ";
+        if (doff[size_t(o)] >= 0) return "dsm[" + std::to_string(doff[size_t(o)]) + " + ";
+        return "p.m[" + std::to_string(int(a.ops[o].moff)) + " + ";
+    };
+    const unsigned hoff_n = (1u << H) < 2u ? 2u : (1u << H);  // a 16-byte multiple
+    // One tile buffer instead of two (kernels only): the next tile is fetched
+    // after this one's stores, and the smaller footprint lets more CTAs share
+    // an SM, whose loads and arithmetic overlap.  Measured on the 30-qubit
+    // spread circuit (B200): complex128 k = 10 316.7 -> 297.5 ms (8 instead of
+    // 6 CTAs per SM), complex64 k = 11 213.6 -> 226.8 ms; so the default is
+    // single for complex128 and double for complex64.  QS_JIT_SINGLE_BUFFER=0/1
+    // overrides it.
+    const bool single = devfn == nullptr && jit_single_buffer(C128);
+    const int nbuf = single ? 1 : 2;
+    out.threads = threads;
+    out.smem = sizeof(V) * size_t(nbuf) * (size_t(1) << K) + 8 * size_t(hoff_n) +
+               (a.nexp > 0 ? sizeof(double2) * size_t(nwarps) * size_t(a.nexp) : 0) +
+               (batched ? sizeof(V) * size_t(NM) : 0) + sizeof(V) * size_t(ndsm);
+    out.smem = (out.smem + 15) & ~size_t(15);
+    // a device function keeps its parameter block in shared memory behind the
+    // rest (see its prologue); the kernels read theirs from the parameter bank
+    const size_t smem_main = out.smem;
+    if (devfn) out.smem += 8 * out.params.size();
+    if (!with_source) return true;
+    const char* VT = C128 ? "double2" : "float2";
+    const char* ST = C128 ? "double" : "float";
+    const char* MK = C128 ? "make_double2" : "make_float2";
+    const char* FMA = C128 ? "__fma_rn" : "__fmaf_rn";
+    // resident threads per SM the register budget is sized for (launch bounds);
+    // QS_JIT_THREADS_PER_SM overrides it
+    static const int env_target = [] {
+        const char* e = getenv("QS_JIT_THREADS_PER_SM");
+        return e && *e ? atoi(e) : 0;
+    }();
+    // 512 threads per SM; plain complex64 state-vector passes (no per-instance
+    // tables, no EXPECT ops) 256, i.e. the whole register file for 64-thread
+    // CTAs: on the 30-qubit spread circuit (B200, k = 11) 211.6 -> 189.7 ms
+    // (384: 208.2 ms).  complex128 passes are fastest at 512 (298 ms at 640,
+    // 344 ms at 768).
+    const int target = env_target > 0 ? env_target : (!C128 && !batched && a.nexp == 0 ? 256 : 512);
+    const int minb = threads >= target ? 1 : target / threads;
+    SrcBuf g;
+    g.add("// generated fused pass: n=%d K=%d L=%d R=%d stages=%d ops=%d expect=%d batched=%d\n", a.n, K, L, R,
+          a.nstages, a.nops, a.nexp, int(batched));
+    g.add("typedef unsigned long long u64;\ntypedef unsigned int u32;\ntypedef %s V;\ntypedef %s S;\n", VT, ST);
+    g.add("static __device__ __forceinline__ V cmul(V a, V b) { V r; r.x = a.x * b.x - a.y * b.y; "
+          "r.y = a.x * b.y + a.y * b.x; return r; }\n");
+    g.add("static __device__ __forceinline__ V cfma(V a, V b, V c) { V r; r.x = %s(a.x, b.x, %s(-a.y, b.y, c.x)); "
+          "r.y = %s(a.x, b.y, %s(a.y, b.x, c.y)); return r; }\n", FMA, FMA, FMA, FMA);
+    g.add("static __device__ __forceinline__ V cadd(V a, V b) { V r; r.x = a.x + b.x; r.y = a.y + b.y; return r; }\n");
+    g.add("static __device__ __forceinline__ V cneg(V a) { V r; r.x = -a.x; r.y = -a.y; return r; }\n");
+    g.add("static __device__ __forceinline__ V csel(bool c, V a, V b) { V r; r.x = c ? a.x : b.x; "
+          "r.y = c ? a.y : b.y; return r; }\n");
+    // products with a real entry a (rmul / rfma) or an imaginary one i*b (imul / ifma)
+    g.add("static __device__ __forceinline__ V rmul(S a, V v) { V r; r.x = a * v.x; r.y = a * v.y; return r; }\n");
+    g.add("static __device__ __forceinline__ V rfma(S a, V v, V c) { V r; r.x = %s(a, v.x, c.x); "
+          "r.y = %s(a, v.y, c.y); return r; }\n", FMA, FMA);
+    g.add("static __device__ __forceinline__ V imul(S b, V v) { V r; r.x = -b * v.y; r.y = b * v.x; return r; }\n");
+    g.add("static __device__ __forceinline__ V ifma(S b, V v, V c) { V r; r.x = %s(-b, v.y, c.x); "
+          "r.y = %s(b, v.x, c.y); return r; }\n", FMA, FMA);
+    g.add("struct __align__(16) P { V m[%d]; u64 ntiles; u64 gthr[8]; u64 gslot[%d]; u64 hibit[16]; u64 gctrl[%d]; "
+          "u64 hsh[%d]; u64 mgoff[%d]; u64 mstride[%d]; u64 eslot[%d]; u64 misc[2];%s };\n", NM, E, NOPS, 4 * NOPS,
+          NOPS, NOPS, NEXP, batched ? (" u32 pe[" + std::to_string(NM) + "];").c_str() : "");
+    // cooperative loops (no per-thread layout): all threads of the CTA
+    const std::string CT = devfn ? "threadIdx.x" : "tid";
+    const std::string CS = devfn ? "blockDim.x" : std::to_string(threads) + "u";
+    if (devfn) {
+        g.add("extern \"C\" __device__ void %s(V* __restrict__ vec, const void* __restrict__ pv, "
+              "const V* __restrict__ mats, double* __restrict__ partials, u64 tile, const u64 tend, "
+              "const u32 zero_in) {\n", devfn);
+    } else {
+        g.add("extern \"C\" __global__ void __launch_bounds__(%d, %d) qs_pass(V* __restrict__ vec, "
+              "const __grid_constant__ P p, const V* __restrict__ mats, double* __restrict__ partials) {\n", threads,
+              minb);
+    }
+    g.add("  extern __shared__ __align__(16) unsigned char smem_raw[];\n");
+    if (devfn) {
+        // the parameter block moves from the plan (global memory) to shared
+        // memory behind the tile buffers: matrix entries are read at shared-
+        // memory latency, as the kernels read them from the constant bank
+        g.add("  { const uint4* __restrict__ src = reinterpret_cast<const uint4*>(pv);\n"
+              "    uint4* dst = reinterpret_cast<uint4*>(smem_raw + %zuu);\n"
+              "    for (u32 i = threadIdx.x; i < %zuu; i += blockDim.x) dst[i] = src[i]; }\n"
+              "  __syncthreads();\n  const P& p = *reinterpret_cast<const P*>(smem_raw + %zuu);\n",
+              smem_main, out.params.size() / 2, smem_main);
+    }
+    g.add("  V* const b0 = reinterpret_cast<V*>(smem_raw);\n  V* const b1 = b0 + %du;\n", single ? 0u : 1u << K);
+    g.add("  u64* const hoff = reinterpret_cast<u64*>(b1 + %du);\n", 1u << K);
+    g.add("  double2* const ered = reinterpret_cast<double2*>(hoff + %du);\n", hoff_n);
+    g.add("  V* const msm = reinterpret_cast<V*>(ered + %d);\n", a.nexp > 0 ? nwarps * a.nexp : 0);
+    g.add("  V* const dsm = msm + %d;\n", batched ? NM : 0);
+    if (devfn) g.add("  const u32 tid = threadIdx.x & %du;\n  const bool act = threadIdx.x < %du;\n",
+                     unsigned(threads - 1), unsigned(threads));
+    else g.add("  const u32 tid = threadIdx.x;\n");
+    g.add("  for (u32 j = %s; j < %du; j += %s) { u64 o = 0;\n", CT.c_str(), 1u << H, CS.c_str());
+    g.add("#pragma unroll\n    for (int t = 0; t < %d; ++t) if ((j >> t) & 1u) o |= p.hibit[t];\n    hoff[j] = o; }\n", H);
+    for (int o = 0; o < a.nops; ++o)
+        if (doff[size_t(o)] >= 0)
+            g.add("  for (u32 q = %s; q < %du; q += %s) dsm[%d + q] = p.m[%d + q];\n", CT.c_str(), 1u << a.cp[o].m,
+                  CS.c_str(), doff[size_t(o)], int(a.ops[o].moff));
+    g.add("  u64 gthr = 0;\n");
+    for (int i = 0; i < nT; ++i) g.add("  if ((tid >> %d) & 1u) gthr |= p.gthr[%d];\n", i, i);
+    for (int si = 0; si < a.nstages; ++si) {
+        const KStage& S = a.st[si];
+        uint32_t rt[8], wt[8], tb[8];
+        for (int i = 0; i < 8; ++i) {
+            rt[i] = S.rthr[i];
+            wt[i] = S.wthr[i];
+            tb[i] = S.tbit[i];
+        }
+        g.add("  const u32 RD%d = %s;\n", si, thread_xor_expr(rt, nT).c_str());
+        if (si > 0) g.add("  const u32 WR%d = %s;\n", si, thread_xor_expr(wt, nT).c_str());
+        g.add("  const u32 TH%d = %s;\n", si, thread_xor_expr(tb, nT).c_str());
+    }
+    g.add("  const u64 ntiles = p.ntiles;\n");
+    g.add("  auto tile_base = [&](u64 t) -> u64 { u64 b = t << %d;\n", L);
+    g.add("#pragma unroll\n    for (int i = 0; i < %d; ++i) { const u64 lo = p.hibit[i] - 1ull; "
+          "b = ((b & ~lo) << 1) | (b & lo); }\n    return b; };\n", H);
+    if (devfn) {  // the caller's tile range
+        g.add("  const u64 tstep = 1;\n");
+        if (batched) g.add("  u64 staged = ~0ull;\n");
+    } else if (batched) {
+        // per-instance tables: contiguous runs of tiles per CTA, so that a CTA
+        // restages its instance's matrices once per instance
+        g.add("  const u64 chunk = (ntiles + gridDim.x - 1) / gridDim.x;\n");
+        g.add("  u64 tile = u64(blockIdx.x) * chunk;\n  const u64 tend = tile + chunk < ntiles ? tile + chunk : ntiles;\n");
+        g.add("  const u64 tstep = 1;\n  u64 staged = ~0ull;\n");
+    } else {
+        g.add("  u64 tile = blockIdx.x;\n  const u64 tend = ntiles;\n  const u64 tstep = gridDim.x;\n");
+    }
+    g.add("  __syncthreads();\n");
+    const int EPC = 16 / int(sizeof(V));
+    g.add("  auto prefetch = [&](V* dst, u64 base) {\n");
+    if (devfn)
+        g.add("    if (zero_in) { for (u32 e = threadIdx.x; e < %du; e += blockDim.x) { V z; z.x = (base == 0 && e == 0) "
+              "? 1 : 0; z.y = 0; dst[e] = z; } } else\n", 1u << K);
+    g.add("    for (u32 c = %s; c < %du; c += %s) { const u32 e = c * %du;\n", CT.c_str(), (1u << K) / EPC, CS.c_str(),
+          EPC);
+    g.add("      const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(dst + e));\n");
+    g.add("      asm volatile(\"cp.async.cg.shared.global [%%0], [%%1], 16;\\n\" :: \"r\"(sa), "
+          "\"l\"(vec + (base | hoff[e >> %d] | (e & %du))) : \"memory\"); }\n", L, (1u << L) - 1u);
+    g.add("    asm volatile(\"cp.async.commit_group;\\n\" ::: \"memory\"); };\n");
+    g.add("  if (tile < tend) prefetch(b0, tile_base(tile));\n");
+    g.add("  for (u32 it = 0; tile < tend; ++it, tile += tstep) {\n");
+    g.add("    V* const cur = (it & 1u) ? b1 : b0;\n    const u64 base = tile_base(tile);\n");
+    g.add("    asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");\n    __syncthreads();\n");
+    if (!single) g.add("    if (tile + tstep < tend) prefetch((it & 1u) ? b0 : b1, tile_base(tile + tstep));\n");
+    if (batched) {
+        g.add("    { const u64 inst = (base & p.misc[0]) >> p.misc[1];\n");
+        g.add("      if (inst != staged) {\n");
+        g.add("        for (u32 q = %s; q < %du; q += %s) { const u32 v = p.pe[q];\n", CT.c_str(), unsigned(a.nmats),
+              CS.c_str());
+        g.add("          if (v >> 31) { const u32 o = (v >> 16) & 0x7fffu; "
+              "msm[q] = mats[p.mgoff[o] + inst * p.mstride[o] + (v & 0xffffu)]; } }\n");
+        g.add("        staged = inst;\n        __syncthreads();\n      } }\n");
+    }
+    // ---- body
+    int fresh = 0;
+    std::vector<int> var(E);  // slot -> SSA value id
+    auto vname = [&](int id) { return "v" + std::to_string(id); };
+    auto slot_addr = [&](const uint16_t* img, int s) {
+        uint32_t c = 0;
+        for (int j = 0; j < R; ++j)
+            if ((s >> j) & 1) c ^= img[j];
+        return c;
+    };
+    // the sum over the nonzero entries of one row of a (slot-order) matrix
+    auto row_expr = [&](int o, int base_idx, int D, const int* in) -> std::string {
+        std::string e;
+        for (int c = 0; c < D; ++c) {
+            const int idx = base_idx + c;
+            const int cl = vclass(o, idx);
+            if (cl == 0) continue;
+            const std::string x = vname(in[c]);
+            const std::string m = mref(o, idx);
+            if (e.empty()) {
+                if (cl == 1) e = x;
+                else if (cl == 2) e = "cneg(" + x + ")";
+                else if (cl == 4) e = "rmul(" + m + ".x, " + x + ")";
+                else if (cl == 5) e = "imul(" + m + ".y, " + x + ")";
+                else e = "cmul(" + m + ", " + x + ")";
+            } else {
+                if (cl == 1) e = "cadd(" + e + ", " + x + ")";
+                else if (cl == 2) e = "cadd(" + e + ", cneg(" + x + "))";
+                else if (cl == 4) e = "rfma(" + m + ".x, " + x + ", " + e + ")";
+                else if (cl == 5) e = "ifma(" + m + ".y, " + x + ", " + e + ")";
+                else e = "cfma(" + m + ", " + x + ", " + e + ")";
+            }
+        }
+        if (e.empty()) e = std::string(MK) + "(0, 0)";
+        return e;
+    };
+    // thread-dependent / outside-tile index bits of a diagonal (h), as an expression
+    auto h_expr = [&](const KOp& op, int o, int si) -> std::string {
+        std::string h;
+        for (int q = 0; q < op.nh; ++q) {
+            const int src = op.hsrc[q];
+            const std::string t = src < 64 ? "((TH" + std::to_string(si) + " >> " + std::to_string(src) + ") & 1u)"
+                                            : "u32((base >> p.hsh[" + std::to_string(4 * o + q) + "]) & 1ull)";
+            h = h.empty() ? t : "((" + h + ") << 1) | " + t;
+        }
+        return h;
+    };
+    for (int s = 0; s < E; ++s) {
+        var[s] = fresh++;
+        g.add("    const V v%d = cur[RD0 ^ %uu];\n", var[s], slot_addr(a.st[0].rslot, s));
+    }
+    for (int si = 0; si < a.nstages; ++si) {
+        const KStage& S = a.st[si];
+        if (si > 0) {
+            g.add("    __syncthreads();\n");
+            for (int s = 0; s < E; ++s) g.add("    cur[WR%d ^ %uu] = v%d;\n", si, slot_addr(S.wslot, s), var[s]);
+            g.add("    __syncthreads();\n");
+            for (int s = 0; s < E; ++s) {
+                var[s] = fresh++;
+                g.add("    const V v%d = cur[RD%d ^ %uu];\n", var[s], si, slot_addr(S.rslot, s));
+            }
+        }
+        for (int o = S.op_begin; o < S.op_begin + S.op_count; ++o) {
+            const KOp& op = a.ops[o];
+            std::string cond;
+            if (op.gctrl) cond = "((base & p.gctrl[" + std::to_string(o) + "]) == p.gctrl[" + std::to_string(o) + "])";
+            if (op.tctrl) {
+                const std::string tc = std::to_string(unsigned(op.tctrl)) + "u";
+                cond += (cond.empty() ? "" : " && ") + std::string("((TH") + std::to_string(si) + " & " + tc +
+                        ") == " + tc + ")";
+            }
+            const int scm = op.scm;
+            auto ctrl_ok = [&](int s) { return (s & scm) == scm; };
+            if (!cond.empty() && op.code != QS_OP_EXPECT) g.add("    const bool c%d = %s;\n", o, cond.c_str());
+            if (op.code == QS_OP_MAT) {
+                const int mask = op.mask, M = popc_c(mask), D = 1 << M;
+                g.add("    // op %d: dense on slot mask %d\n", o, mask);
+                for (int s = 0; s < E; ++s) {
+                    if ((s & mask) || !ctrl_ok(s)) continue;
+                    int in[16], outid[16];
+                    for (int c = 0; c < D; ++c) in[c] = var[s | pdep_c(c, mask)];
+                    for (int r = 0; r < D; ++r) {
+                        const std::string e = row_expr(o, op.moff + r * D, D, in);
+                        outid[r] = fresh++;
+                        if (cond.empty()) g.s += "    const V " + vname(outid[r]) + " = " + e + ";\n";
+                        else g.s += "    const V " + vname(outid[r]) + " = c" + std::to_string(o) + " ? " + e + " : " +
+                                    vname(in[r]) + ";\n";
+                    }
+                    for (int r = 0; r < D; ++r) var[s | pdep_c(r, mask)] = outid[r];
+                }
+            } else if (op.code == QS_OP_ANTI || op.code == QS_OP_SWAP) {  // plain exchanges
+                int b0, b1;
+                if (op.code == QS_OP_ANTI) {
+                    b0 = 0;
+                    b1 = op.mask;
+                } else {
+                    b0 = 1 << nth_bit(op.mask, 0);
+                    b1 = 1 << nth_bit(op.mask, 1);
+                }
+                for (int s = 0; s < E; ++s) {
+                    if ((s & op.mask) || !ctrl_ok(s)) continue;
+                    const int x0 = var[s | b0], x1 = var[s | b1];
+                    if (cond.empty()) {
+                        var[s | b0] = x1;
+                        var[s | b1] = x0;
+                    } else {
+                        const int n0 = fresh++, n1 = fresh++;
+                        g.add("    const V v%d = csel(c%d, v%d, v%d);\n", n0, o, x1, x0);
+                        g.add("    const V v%d = csel(c%d, v%d, v%d);\n", n1, o, x0, x1);
+                        var[s | b0] = n0;
+                        var[s | b1] = n1;
+                    }
+                }
+            } else if (op.code == QS_OP_DIAG) {
+                g.add("    // op %d: diagonal, %d register bits, %d other bits\n", o, op.ns, op.nh);
+                if (op.nh > 0) g.s += "    const u32 h" + std::to_string(o) + " = " + h_expr(op, o, si) + ";\n";
+                for (int s = 0; s < E; ++s) {
+                    if (!ctrl_ok(s)) continue;
+                    const int k = op.kidx[s];
+                    std::string e;
+                    if (op.nh == 0) {
+                        const int idx = op.moff + k;
+                        const int cl = vclass(o, idx);
+                        if (cl == 1) continue;
+                        if (cl == 2) e = "cneg(" + vname(var[s]) + ")";
+                        else if (cl == 0) e = std::string(MK) + "(0, 0)";
+                        else if (cl == 4) e = "rmul(" + mref(o, idx) + ".x, " + vname(var[s]) + ")";
+                        else if (cl == 5) e = "imul(" + mref(o, idx) + ".y, " + vname(var[s]) + ")";
+                        else e = "cmul(" + vname(var[s]) + ", " + mref(o, idx) + ")";
+                    } else {
+                        e = "cmul(" + vname(var[s]) + ", " + dtab(o) + "((h" + std::to_string(o) + " << " +
+                            std::to_string(int(op.ns)) + ") | " + std::to_string(k) + "u)])";
+                    }
+                    const int nid = fresh++;
+                    if (cond.empty()) g.s += "    const V " + vname(nid) + " = " + e + ";\n";
+                    else g.s += "    const V " + vname(nid) + " = c" + std::to_string(o) + " ? " + e + " : " +
+                                vname(var[s]) + ";\n";
+                    var[s] = nid;
+                }
+            } else if (op.code == QS_OP_EXPECT) {
+                // sum over the thread's psi/lam pairs (slot bit 0 = pair bit) of
+                // conj(lam) (G psi) in the state's precision, then a warp sum in FP64
+                if (!cond.empty() || scm != 0 || pair_tile < 0 || S.R[0] != pair_tile) return false;
+                g.add("    { // op %d: <lam| G |psi>\n      S pr = 0, pi = 0;\n", o);
+                const bool dg = op.flags & QS_OPF_DIAG;
+                if (dg && op.nh > 0) g.s += "      const u32 h" + std::to_string(o) + " = " + h_expr(op, o, si) + ";\n";
+                if (dg) {
+                    for (int s = 0; s < E; s += 2) {
+                        const int k = op.kidx[s];
+                        std::string d = op.nh == 0 ? mref(o, op.moff + k)
+                                                   : dtab(o) + "((h" + std::to_string(o) + " << " +
+                                                         std::to_string(int(op.ns)) + ") | " + std::to_string(k) +
+                                                         "u)]";
+                        g.s += "      { const V acc = cmul(" + d + ", " + vname(var[s]) + "); const V l = " +
+                               vname(var[s | 1]) + ";\n";
+                        g.s += "        pr += l.x * acc.x + l.y * acc.y; pi += l.x * acc.y - l.y * acc.x; }\n";
+                    }
+                } else {
+                    const int mask = op.mask, M = popc_c(mask), D = 1 << M;
+                    if ((mask & 1) || M > 2) return false;
+                    for (int s = 0; s < E; ++s) {
+                        if ((s & mask) || (s & 1)) continue;
+                        int in[4];
+                        for (int c = 0; c < D; ++c) in[c] = var[s | pdep_c(c, mask)];
+                        for (int r = 0; r < D; ++r) {
+                            g.s += "      { const V acc = " + row_expr(o, op.moff + r * D, D, in) + "; const V l = " +
+                                   vname(var[s | 1 | pdep_c(r, mask)]) + ";\n";
+                            g.s += "        pr += l.x * acc.x + l.y * acc.y; pi += l.x * acc.y - l.y * acc.x; }\n";
+                        }
+                    }
+                }
+                g.add("      double re = pr, im = pi;\n");
+                g.add("#pragma unroll\n      for (int off = 16; off > 0; off >>= 1) { re += __shfl_xor_sync(0xffffffffu, "
+                      "re, off); im += __shfl_xor_sync(0xffffffffu, im, off); }\n");
+                g.add("      if ((tid & 31u) == 0) ered[(tid >> 5) * %d + %d] = make_double2(re, im);\n    }\n", NEXP,
+                      int(op.elocal));
+            } else {
+                return false;
+            }
+        }
+    }
+    if (devfn) g.add("    if (act) {\n");
+    for (int s = 0; s < E; ++s) g.add("    vec[base | gthr | p.gslot[%d]] = v%d;\n", s, var[s]);
+    if (devfn) g.add("    }\n");
+    if (a.nexp > 0) {
+        // per-tile partials: the warps' sums in a fixed order
+        g.add("    __syncthreads();\n");
+        g.add("    for (u32 e = %s; e < %du; e += %s) { double2 t = make_double2(0.0, 0.0);\n", CT.c_str(),
+              unsigned(a.nexp), CS.c_str());
+        g.add("      for (int w = 0; w < %d; ++w) { t.x += ered[w * %d + e].x; t.y += ered[w * %d + e].y; }\n", nwarps,
+              NEXP, NEXP);
+        g.add("      const u64 at = 2 * (p.eslot[e] * ntiles + tile);\n      partials[at] = t.x;\n"
+              "      partials[at + 1] = t.y; }\n");
+    }
+    if (single)  // every thread is past its last read of the buffer
+        g.add("    __syncthreads();\n    if (tile + tstep < tend) prefetch(b0, tile_base(tile + tstep));\n");
+    g.add("  }\n}\n");
+    if (g.truncated) return false;
+    out.src.swap(g.s);
+    return true;
+}
+
+}  // namespace
+
+bool gen_pass(const void* regargs, int R, bool c128, const void* mats_host, JitPass& out, bool with_source,
+              const char* devfn) {
+    const RegArgs& a = *static_cast<const RegArgs*>(regargs);
+    return c128 ? gen_reg_pass<double2>(a, R, static_cast<const double2*>(mats_host), out, with_source, devfn)
+                : gen_reg_pass<float2>(a, R, static_cast<const float2*>(mats_host), out, with_source, devfn);
+}
+
+bool gen_batch_pass(const void* regargs, int R, bool c128, const void* mats_host, const char* name, std::string* src,
+                    std::vector<uint64_t>* params, size_t* smem, int* threads) {
+    JitPass jp;
+    if (!gen_pass(regargs, R, c128, mats_host, jp, true, name)) return false;
+    src->swap(jp.src);
+    params->swap(jp.params);
+    *smem = jp.smem;
+    *threads = jp.threads;
+    return true;
+}
+
+}  // namespace qs
