@@ -11,6 +11,8 @@
 // share one compiled kernel (jit.cu caches by source text).
 #include <algorithm>
 #include <array>
+#include <cmath>
+#include <complex>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -64,6 +66,307 @@ std::string thread_xor_expr(const uint32_t* img, int nT) {
     }
     return e.empty() ? std::string("0u") : e;
 }
+
+// ---------------------------------------------------------------- normalised matrices
+// What bounds a pass over a large state is its multiply-add count, and most of
+// its dense matrices are known only up to factors that need not be applied
+// where they stand.  A dense matrix U is written as U = s (D_1 x D_2) U' with a
+// scalar s and a diagonal D_i = diag(1, d_i) per target bit, chosen so that the
+// diagonal entries of U' are exactly 1 (row r's factor is s times the d_i of
+// its set index bits): an entry 1 costs nothing where a general one costs four
+// instructions per amplitude, a real or imaginary one two.
+//   - s commutes with everything: the launch's scalars are multiplied into one
+//     uncontrolled op (the one whose cost grows least).
+//   - D_i moves forward along its bit (through diagonals and controls, across
+//     plain exchanges) into the next uncontrolled op on that bit; d_i = 1 when
+//     no op takes it.
+// Row and scalar factors leave every product's relative rounding error as it
+// is; only the range grows, so the launch's factors are bounded (see run).
+// Which entry becomes 1 depends on the pattern of zeros and on classes that
+// hold for every value (real, imaginary, equal up to sign), not on the values'
+// sizes: new parameters of a circuit reuse its compiled kernels.
+// 30-qubit spread circuit of 1000 gates (B200): 3316 -> 2706 multiply-add
+// instructions per amplitude, complex128 318.3 -> 276.3 ms, complex64 202.4 ->
+// 179.0 ms; 25 qubits, 300 gates, complex64 2.04 -> 1.84 ms, its error against
+// 64-bit arithmetic 3.8e-7 -> 3.5e-7 (fewer roundings).  Per-instance tables
+// and adjoint passes keep their matrices.
+using Cx = std::complex<double>;
+
+// 0, 1, -1, general (3), real (4), imaginary (5)
+template <typename T>
+int value_class(T x, T y) {
+    if (y == 0) return x == 0 ? 0 : x == 1 ? 1 : x == -1 ? 2 : 4;
+    return x == 0 ? 5 : 3;
+}
+
+// Instructions per amplitude of one row: the first term may be a unit entry
+// (taken as is), which the generated code puts first.
+int row_cost(const Cx* m, int D) {
+    int c = 0;
+    bool unit = false, any = false;
+    for (int i = 0; i < D; ++i) {
+        const int cl = value_class(m[i].real(), m[i].imag());
+        if (cl == 0) continue;
+        any = true;
+        if (cl <= 2) unit = true;
+        c += cl == 3 ? 4 : 2;
+    }
+    return any && unit ? c - 2 : c;
+}
+int mat_cost(const Cx* m, int D) {  // summed over the rows
+    int c = 0;
+    for (int r = 0; r < D; ++r) c += row_cost(m + r * D, D);
+    return c;
+}
+
+// Products and quotients that keep the classes: exact zeros stay, and a part
+// that vanishes, or a quotient that is +-1, up to the rounding of this very
+// operation is what it is for every value (a phase that cancels), so it is set;
+// a class that came and went with the last bit would mean another kernel.
+constexpr double kClassTol = 0x1p-48;
+Cx settle(Cx q) {
+    const double r = std::abs(q.real()), i = std::abs(q.imag());
+    if (i <= kClassTol * r) return Cx(q.real(), 0.0);
+    if (r <= kClassTol * i) return Cx(0.0, q.imag());
+    return q;
+}
+Cx exact_mul(Cx a, Cx b) {
+    if (a.imag() == 0 && b.imag() == 0) return Cx(a.real() * b.real(), 0.0);
+    return settle(Cx(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()));
+}
+Cx exact_div(Cx a, Cx b) {
+    if (a == b) return Cx(1, 0);
+    if (a == -b) return Cx(-1, 0);
+    if (a == Cx(0, 0)) return Cx(0, 0);
+    const Cx q = b.imag() == 0 ? Cx(a.real() / b.real(), a.imag() / b.real()) : settle(a / b);
+    if (q.imag() == 0 && std::abs(std::abs(q.real()) - 1.0) <= kClassTol) return Cx(q.real() > 0 ? 1 : -1, 0);
+    return q;
+}
+
+struct Normaliser {
+    const RegArgs& a;
+    std::vector<std::vector<Cx>>& m;  // per op, slot order (MAT: row-major D x D; DIAG: 2^m entries)
+    // log2 bounds on how far taking factors out may raise (up) and lower (down)
+    // the amplitudes between the launch's load and its store
+    const double max_up, max_down;
+
+    Normaliser(const RegArgs& a_, std::vector<std::vector<Cx>>& m_, double max_up_, double max_down_)
+        : a(a_), m(m_), max_up(max_up_), max_down(max_down_) {}
+
+    const KStage& stage_of(int o) const {
+        for (int si = 0; si < a.nstages; ++si)
+            if (o < a.st[si].op_begin + a.st[si].op_count) return a.st[si];
+        return a.st[a.nstages - 1];
+    }
+    static bool controlled(const KOp& op) { return op.scm || op.tctrl || op.gctrl; }
+    // index bit of tile bit b among op o's targets, or -1
+    int index_bit(int o, int b) const {
+        const KOp& op = a.ops[o];
+        const KStage& S = stage_of(o);
+        int i = 0;
+        for (int j = 0; j < 6; ++j) {
+            if (!((op.mask >> j) & 1)) continue;
+            if (S.R[j] == b) return i;
+            ++i;
+        }
+        if (op.code == QS_OP_DIAG)
+            for (int q = 0; q < op.nh; ++q)
+                if (op.hsrc[q] == b) return op.ns + (op.nh - 1 - q);
+        return -1;
+    }
+    // a diagonal whose every entry is multiplied anyway takes factors for free
+    bool free_diag(int o) const {
+        const KOp& op = a.ops[o];
+        if (op.code != QS_OP_DIAG || controlled(op)) return false;
+        if (op.nh > 0) return true;
+        for (const Cx& z : m[size_t(o)])
+            if (value_class(z.real(), z.imag()) != 3) return false;
+        return true;
+    }
+    // The op that takes a factor diag(1, d) of tile bit b from op o, the bit it
+    // then sits on, and whether an odd number of exchanges inverts it; -1: none.
+    int taker(int o, int b, int* bit, bool* inverted) const {
+        *inverted = false;
+        for (int p = o + 1; p < a.nops; ++p) {
+            const KOp& op = a.ops[p];
+            const int ib = index_bit(p, b);
+            if (ib < 0) continue;
+            if (op.code == QS_OP_DIAG) {
+                if (!free_diag(p)) continue;
+            } else if (controlled(op)) {
+                return -1;
+            } else if (op.code == QS_OP_ANTI) {
+                *inverted = !*inverted;
+                continue;
+            } else if (op.code == QS_OP_SWAP) {
+                const KStage& S = stage_of(p);
+                const int b0 = S.R[nth_bit(op.mask, 0)], b1 = S.R[nth_bit(op.mask, 1)];
+                b = b == b0 ? b1 : b0;
+                continue;
+            } else if (op.code != QS_OP_MAT) {
+                return -1;
+            }
+            *bit = b;
+            return p;
+        }
+        return -1;
+    }
+    // m[p] <- m[p] diag(1, d) on index bit ib (columns; entries of a diagonal)
+    void take(std::vector<Cx>& v, bool diag, int ib, Cx d) const {
+        const size_t D = diag ? v.size() : size_t(1) << (ctz(v.size()) / 2);
+        for (size_t e = 0; e < v.size(); ++e)
+            if (((e & (D - 1)) >> ib) & 1) v[e] = exact_mul(v[e], d);
+    }
+    static int ctz(size_t x) {
+        int c = 0;
+        while (!((x >> c) & 1)) ++c;
+        return c;
+    }
+    // best cost of a matrix whose rows may all be scaled (an estimate)
+    static int scaled_cost(std::vector<Cx> v) {
+        const int D = 1 << (ctz(v.size()) / 2);
+        for (int r = 0; r < D; ++r) {
+            const Cx z = v[size_t(r * D + r)];
+            if (D > 4 || z == Cx(0, 0)) continue;
+            for (int c = 0; c < D; ++c) v[size_t(r * D + c)] = exact_div(v[size_t(r * D + c)], z);
+        }
+        return mat_cost(v.data(), D);
+    }
+
+    // Take factors out of every uncontrolled dense op on one or two bits.
+    void run() {
+        Cx total(1, 0);
+        double up = 0, down = 0, held = 0;                 // scalars so far; factors on their way to a taker
+        std::vector<double> raised(size_t(a.nops), 0.0);  // by the scalar taken out of each op
+        std::vector<double> release(size_t(a.nops), 0.0);
+        for (int o = 0; o < a.nops; ++o) {
+            held -= release[size_t(o)];
+            const KOp& op = a.ops[o];
+            if (op.code != QS_OP_MAT || controlled(op)) continue;
+            std::vector<Cx>& u = m[size_t(o)];
+            const int M = popc_c(op.mask), D = 1 << M;
+            if (M > 2) continue;
+            const KStage& S = stage_of(o);
+            const Cx s = u[0];
+            if (!usable(s, u)) continue;
+            std::vector<Cx> d(size_t(M), Cx(1, 0));
+            std::vector<Cx> best = scaled(u, s, d);
+            int best_cost = mat_cost(best.data(), D);
+            const double ls = std::log2(std::abs(s));
+            const double u_up = std::max(0.0, -ls), u_down = std::max(0.0, ls);
+            double u_held = 0;
+            if (best_cost >= mat_cost(u.data(), D)) continue;
+            std::vector<int> to(size_t(M), -1), tob(size_t(M), 0);
+            std::vector<char> inv(size_t(M), 0);
+            for (int i = 0; i < M; ++i) {
+                const Cx z = u[size_t((1 << i) * D + (1 << i))];
+                if (!usable(z, u)) continue;
+                bool iv = false;
+                int bit = 0;
+                const int p = taker(o, S.R[nth_bit(op.mask, i)], &bit, &iv);
+                if (p < 0) continue;
+                std::vector<Cx> d2 = d;
+                d2[size_t(i)] = exact_div(z, s);
+                if (d2[size_t(i)] == Cx(1, 0)) continue;
+                const std::vector<Cx> v = scaled(u, s, d2);
+                // per amplitude: this op gains, a dense taker may lose
+                double gain = double(best_cost - mat_cost(v.data(), D)) / D;
+                const bool dg = a.ops[p].code == QS_OP_DIAG;
+                if (!dg) {
+                    std::vector<Cx> w = m[size_t(p)];
+                    const int D2 = 1 << (ctz(w.size()) / 2);
+                    const int before = scaled_cost(w);
+                    take(w, false, index_bit(p, bit), d2[size_t(i)]);
+                    gain -= double(scaled_cost(w) - before) / D2;
+                }
+                if (gain <= 0) continue;
+                d = d2;
+                best = v;
+                best_cost = mat_cost(v.data(), D);
+                to[size_t(i)] = p;
+                tob[size_t(i)] = bit;
+                inv[size_t(i)] = iv;
+                u_held += std::abs(std::log2(std::abs(d2[size_t(i)])));
+            }
+            if (up + u_up > max_up || down + u_down + held + u_held > max_down) continue;
+            up += u_up;
+            down += u_down;
+            held += u_held;
+            raised[size_t(o)] = -ls;
+            u = best;
+            total = exact_mul(total, s);
+            for (int i = 0; i < M; ++i) {
+                if (to[size_t(i)] < 0) continue;
+                Cx f = d[size_t(i)];
+                if (inv[size_t(i)]) {  // X diag(1, d) = d diag(1, 1/d) X
+                    total = exact_mul(total, f);
+                    f = exact_div(Cx(1, 0), f);
+                }
+                const int p = to[size_t(i)];
+                release[size_t(p)] += std::abs(std::log2(std::abs(d[size_t(i)])));
+                take(m[size_t(p)], a.ops[p].code == QS_OP_DIAG, index_bit(p, tob[size_t(i)]), f);
+            }
+        }
+        if (total == Cx(1, 0)) return;
+        // The op that carries the scalars: the amplitudes are low from it until
+        // the ops after it have raised them again, by at most max_down.
+        int carrier = -1;
+        double least = 1e300, after = 0;
+        for (int o = a.nops - 1; o >= 0; --o) {
+            const KOp& op = a.ops[o];
+            const double low = after;
+            after += std::max(0.0, raised[size_t(o)]);
+            if (low > max_down) break;
+            if (controlled(op) || (op.code != QS_OP_MAT && op.code != QS_OP_DIAG)) continue;
+            std::vector<Cx> v = m[size_t(o)];
+            for (Cx& z : v) z = exact_mul(z, total);
+            double more;
+            if (op.code == QS_OP_DIAG) {
+                more = op.nh > 0 ? 0.0 : double(diag_cost(v) - diag_cost(m[size_t(o)])) / double(v.size());
+            } else {
+                const int D = 1 << (ctz(v.size()) / 2);
+                more = double(mat_cost(v.data(), D) - mat_cost(m[size_t(o)].data(), D)) / D;
+            }
+            if (more < least) {
+                least = more;
+                carrier = o;
+            }
+        }
+        for (Cx& z : m[size_t(carrier)]) z = exact_mul(z, total);
+    }
+    static int diag_cost(const std::vector<Cx>& v) {
+        int c = 0;
+        for (const Cx& z : v) {
+            const int cl = value_class(z.real(), z.imag());
+            c += cl == 1 ? 0 : cl == 3 ? 4 : 2;
+        }
+        return c;
+    }
+    // a factor that is neither zero nor far below the matrix's largest entry
+    // (then the matrix keeps its own form)
+    static bool usable(Cx z, const std::vector<Cx>& u) {
+        double top = 0;
+        for (const Cx& e : u) top = std::max(top, std::abs(e));
+        const double r = std::abs(z);
+        return r > top * 0x1p-20 && r >= 0x1p-20 && r <= 0x1p20;
+    }
+    // rows divided by s times the d_i of the set index bits
+    static std::vector<Cx> scaled(const std::vector<Cx>& u, Cx s, const std::vector<Cx>& d) {
+        const int M = int(d.size()), D = 1 << M;
+        std::vector<Cx> v(u.size());
+        for (int r = 0; r < D; ++r) {
+            Cx f = s;
+            for (int i = 0; i < M; ++i)
+                if ((r >> i) & 1) f = d[size_t(i)] == Cx(1, 0) ? f : exact_mul(f, d[size_t(i)]);
+            for (int c = 0; c < D; ++c) {
+                // the rows whose factor is their own diagonal entry get an exact 1
+                const bool own = c == r && (r == 0 || ((r & (r - 1)) == 0 && !(d[size_t(ctz(size_t(r)))] == Cx(1, 0))));
+                v[size_t(r * D + c)] = own ? Cx(1, 0) : exact_div(u[size_t(r * D + c)], f);
+            }
+        }
+        return v;
+    }
+};
 
 // devfn != nullptr: emit the pass as `extern "C" __device__ void <devfn>(vec,
 // params, mats, partials, tile, tend, zero_in)` for the persistent batch
@@ -124,6 +427,18 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
         }
     }
     if (a.nops > 32767) return false;
+    if (!batched && a.nexp == 0) {
+        std::vector<std::vector<Cx>> um(static_cast<size_t>(a.nops));
+        for (int o = 0; o < a.nops; ++o) {
+            const KCopy& c = a.cp[o];
+            const int cnt = c.diag ? (1 << c.m) : (1 << (2 * c.m));
+            for (int e = 0; e < cnt; ++e) um[size_t(o)].emplace_back(double(pm[c.soff + e].x), double(pm[c.soff + e].y));
+        }
+        Normaliser(a, um, C128 ? 600.0 : 60.0, C128 ? 300.0 : 24.0).run();
+        for (int o = 0; o < a.nops; ++o)
+            for (size_t e = 0; e < um[size_t(o)].size(); ++e)
+                pm[a.cp[o].soff + e] = mk<V>(um[size_t(o)][e].real(), um[size_t(o)][e].imag());
+    }
     // tile position of the psi/lam pair bit (adjoint pair passes)
     int pair_tile = -1;
     for (int b = 0; b < 64 && a.pairmask; ++b)
@@ -156,15 +471,6 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
     // every instance's value (e.g. real for the entries of Ry tables, imaginary
     // for the off-diagonal entries of Rx tables); the value itself is read from
     // the staged table at run time.
-    auto value_class = [](const V v) -> int {
-        if (v.y == 0) {
-            if (v.x == 0) return 0;
-            if (v.x == 1) return 1;
-            if (v.x == -1) return 2;
-            return 4;
-        }
-        return v.x == 0 ? 5 : 3;
-    };
     auto join_class = [](int c1, int c2) -> int {
         if (c1 == c2) return c1;
         const bool r1 = c1 == 0 || c1 == 1 || c1 == 2 || c1 == 4, r2 = c2 == 0 || c2 == 1 || c2 == 2 || c2 == 4;
@@ -189,12 +495,12 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
                 sc |= ((kc >> i) & 1) << c.perm[i];
             }
             const int64_t src = c.goff + (c.diag ? sr : sr * D + sc);
-            int cl = value_class(hm[src]);
-            for (int64_t i = 1; i < ninst && cl != 3; ++i) cl = join_class(cl, value_class(hm[src + i * c.stride]));
+            int cl = value_class(hm[src].x, hm[src].y);
+            for (int64_t i = 1; i < ninst && cl != 3; ++i) cl = join_class(cl, value_class(hm[src + i * c.stride].x, hm[src + i * c.stride].y));
             scls[size_t(c.soff + e)] = uint8_t(cl);
         }
     }
-    auto vclass = [&](int o, int idx) -> int { return strided[o] ? int(scls[size_t(idx)]) : value_class(pm[idx]); };
+    auto vclass = [&](int o, int idx) -> int { return strided[o] ? int(scls[size_t(idx)]) : value_class(pm[idx].x, pm[idx].y); };
     auto mref = [&](int o, int idx) -> std::string {
         return (strided[o] ? "msm[" : "p.m[") + std::to_string(idx) + "]";
     };
@@ -390,7 +696,11 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
     // the sum over the nonzero entries of one row of a (slot-order) matrix
     auto row_expr = [&](int o, int base_idx, int D, const int* in) -> std::string {
         std::string e;
-        for (int c = 0; c < D; ++c) {
+        int first = 0;  // start from a unit entry: it costs nothing
+        for (int c = D - 1; c >= 0; --c)
+            if (vclass(o, base_idx + c) == 1 || vclass(o, base_idx + c) == 2) first = c;
+        for (int i = 0; i < D; ++i) {
+            const int c = i == 0 ? first : i <= first ? i - 1 : i;
             const int idx = base_idx + c;
             const int cl = vclass(o, idx);
             if (cl == 0) continue;
