@@ -533,12 +533,14 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
     };
     const unsigned hoff_n = (1u << H) < 2u ? 2u : (1u << H);  // a 16-byte multiple
     // One tile buffer instead of two (kernels only): the next tile is fetched
-    // after this one's stores, and the smaller footprint lets more CTAs share
-    // an SM, whose loads and arithmetic overlap.  Measured on the 30-qubit
-    // spread circuit (B200): complex128 k = 10 316.7 -> 297.5 ms (8 instead of
-    // 6 CTAs per SM), complex64 k = 11 213.6 -> 226.8 ms; so the default is
-    // single for complex128 and double for complex64.  QS_JIT_SINGLE_BUFFER=0/1
-    // overrides it.
+    // once the last stage has read this one, under that stage's arithmetic and
+    // stores, and the smaller footprint lets more CTAs share an SM, whose loads
+    // and arithmetic overlap.  Measured on the 30-qubit spread circuit (B200),
+    // one buffer against two: complex128 k = 11 270 against 284 ms, complex64
+    // k = 12 164.6 against 163.2 ms, k = 11 168.3 against 166.1 ms; so the
+    // default is single for complex128 and double for complex64.  Fetching only
+    // after the stores: complex128 k = 12 276 ms, now 261 ms (k = 10: 272, 269).
+    // QS_JIT_SINGLE_BUFFER=0/1 overrides it.
     const bool single = devfn == nullptr && jit_single_buffer(C128);
     const int nbuf = single ? 1 : 2;
     out.threads = threads;
@@ -749,6 +751,8 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
                 g.add("    const V v%d = cur[RD%d ^ %uu];\n", var[s], si, slot_addr(S.rslot, s));
             }
         }
+        if (single && si == a.nstages - 1)  // the buffer's last readers: the next tile comes in under the last stage
+            g.add("    __syncthreads();\n    if (tile + tstep < tend) prefetch(b0, tile_base(tile + tstep));\n");
         for (int o = S.op_begin; o < S.op_begin + S.op_count; ++o) {
             const KOp& op = a.ops[o];
             std::string cond;
@@ -881,8 +885,6 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
         g.add("      const u64 at = 2 * (p.eslot[e] * ntiles + tile);\n      partials[at] = t.x;\n"
               "      partials[at + 1] = t.y; }\n");
     }
-    if (single)  // every thread is past its last read of the buffer
-        g.add("    __syncthreads();\n    if (tile + tstep < tend) prefetch(b0, tile_base(tile + tstep));\n");
     g.add("  }\n}\n");
     if (g.truncated) return false;
     out.src.swap(g.s);
