@@ -24,6 +24,7 @@
 // (statevector_simulator.py:155-164, gate_function.py:31-1031).
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstdarg>
 #include <cstring>
 #include <memory>
@@ -326,6 +327,26 @@ struct JitMemo {
     int occ[64] = {0};
 };
 
+std::mutex& memo_mu() {  // guards the memos and their table
+    static std::mutex mu;
+    return mu;
+}
+std::unordered_map<uint64_t, std::shared_ptr<JitMemo>>& memo_table() {
+    static std::unordered_map<uint64_t, std::shared_ptr<JitMemo>> t;
+    return t;
+}
+std::shared_ptr<JitMemo> get_memo(uint64_t key) {
+    std::lock_guard<std::mutex> lock(memo_mu());
+    auto it = memo_table().find(key);
+    return it == memo_table().end() ? nullptr : it->second;
+}
+// the memo of `key`: `m`, or the one another thread put there first
+std::shared_ptr<JitMemo> put_memo(uint64_t key, std::shared_ptr<JitMemo> m) {
+    std::lock_guard<std::mutex> lock(memo_mu());
+    if (memo_table().size() > 4096) memo_table().clear();  // bounded: plans are cheap to regenerate
+    return memo_table().emplace(key, std::move(m)).first->second;
+}
+
 uint64_t fnv(uint64_t h, const void* p, size_t n) {
     const unsigned char* c = static_cast<const unsigned char*>(p);
     for (size_t i = 0; i < n; ++i) h = (h ^ c[i]) * 1099511628211ull;
@@ -361,54 +382,173 @@ uint64_t plan_key(const RegArgs& a, int R, size_t vsize, const std::vector<uint8
     return fnv(h, classes.data(), classes.size());
 }
 
+// ------------------------------------------------------- plans kept between launches
+// Planning a register pass (build_reg scores every set of R tile bits for
+// every stage) and generating its parameter block take 0.1 - 1 ms of host
+// time, several times what the pass itself takes on a small state.  Both are
+// functions of the pass's description alone, so they are kept: a plan under
+// the exact contents of the pass and its ops, and, per plan, the parameter
+// blocks of the matrix values it last ran with (none for per-instance tables,
+// whose values are read on the device).  Contents are compared in full, and the
+// store is dropped whole when it holds more than kPlanBytes.  run() of a known
+// circuit with the keys of its ops kept as well (B200): 10 qubits, 60 gates
+// 239 -> 81 us; 20 qubits, 200 gates 619 -> 243 us; 25 qubits, 300 gates in
+// complex64 1.84 -> 1.46 ms (the host planned longer than the GPU ran).
+struct ParamSet {
+    std::vector<unsigned char> values;  // the matrix entries the block was made from
+    JitPass jp;
+    uint64_t key = 0;                   // plan_key: structure and value classes
+    std::shared_ptr<JitMemo> memo;
+};
+struct PlanLaunch {
+    RegArgs args;
+    std::vector<int> rem;  // positions of the pass's ops that had not run before this launch
+    std::mutex mu;  // guards sets
+    std::vector<std::shared_ptr<const ParamSet>> sets;
+};
+struct PassPlan {
+    std::vector<unsigned char> content;
+    std::vector<std::unique_ptr<PlanLaunch>> launches;
+};
+constexpr size_t kPlanBytes = size_t(64) << 20;
+constexpr size_t kParamSets = 8;  // per launch
+
+std::mutex g_plan_mu;  // guards the two below
+std::unordered_map<uint64_t, std::shared_ptr<PassPlan>> g_plans;
+std::atomic<size_t> g_plan_bytes{0};
+
+// Word-wise hash of a byte string (the contents themselves are compared).
+uint64_t hash_bytes(uint64_t h, const void* p, size_t n) {
+    const unsigned char* c = static_cast<const unsigned char*>(p);
+    for (; n >= 8; n -= 8, c += 8) {
+        uint64_t w;
+        memcpy(&w, c, 8);
+        h = (h ^ w) * 0x9e3779b97f4a7c15ull;
+        h ^= h >> 29;
+    }
+    return n ? fnv(h, c, n) : h;
+}
+
+// The plan of a pass: every launch it splits into.  nullptr with the error set
+// when an op does not fit.
+std::shared_ptr<PassPlan> get_plan(const qs_pass& ps, const qs_op* ops, int n, int R, int nb) {
+    static thread_local std::vector<unsigned char> content;
+    const int head[] = {n, R, nb, ps.k, ps.nlow, ps.inst_shift, ps.pair, ps.op_count};
+    const size_t hb = sizeof(head), pb = sizeof(ps.hi), ob = sizeof(qs_op) * size_t(ps.op_count);
+    content.resize(hb + pb + ob);
+    memcpy(content.data(), head, hb);
+    memset(content.data() + hb, 0, pb);
+    memcpy(content.data() + hb, ps.hi, sizeof(int32_t) * size_t(ps.k - ps.nlow));
+    memcpy(content.data() + hb + pb, ops + ps.op_begin, ob);
+    const uint64_t key = hash_bytes(1469598103934665603ull, content.data(), content.size());
+    {
+        std::lock_guard<std::mutex> lock(g_plan_mu);
+        auto it = g_plans.find(key);
+        if (it != g_plans.end() && it->second->content == content) return it->second;
+    }
+    auto plan = std::make_shared<PassPlan>();
+    plan->content = content;
+    std::vector<int> rem(ps.op_count);
+    for (int i = 0; i < ps.op_count; ++i) rem[i] = i;
+    while (!rem.empty()) {
+        const int next = ps.op_begin + rem.front();
+        auto L = std::make_unique<PlanLaunch>();
+        L->rem = rem;
+        if (build_reg(ps, ops, rem, n, R, nb, L->args) <= 0) {
+            set_error("qs_apply_fused: op %d does not fit a register tile", next);
+            return nullptr;
+        }
+        plan->launches.push_back(std::move(L));
+    }
+    std::lock_guard<std::mutex> lock(g_plan_mu);
+    if (g_plan_bytes > kPlanBytes) {
+        g_plans.clear();  // plans in use live on with their callers
+        g_plan_bytes = 0;
+    }
+    g_plan_bytes += content.size() + sizeof(PlanLaunch) * plan->launches.size();
+    g_plans[key] = plan;
+    return plan;
+}
+
+// The parameter block of a planned launch for the values in `hm` (kept when
+// the launch has no per-instance tables); nullptr when it is not generated.
+template <typename V>
+std::shared_ptr<const ParamSet> get_params(PlanLaunch& L, int R, const V* hm) {
+    const RegArgs& a = L.args;
+    static thread_local std::vector<unsigned char> values;
+    values.clear();
+    if (!a.batched) {
+        for (int o = 0; o < a.nops; ++o) {
+            const KCopy& c = a.cp[o];
+            const size_t cnt = size_t(1) << (c.diag ? c.m : 2 * c.m);
+            const unsigned char* p = reinterpret_cast<const unsigned char*>(hm + c.goff);
+            values.insert(values.end(), p, p + cnt * sizeof(V));
+        }
+        std::lock_guard<std::mutex> lock(L.mu);
+        for (const auto& s : L.sets)
+            if (s->values == values) return s;
+    }
+    auto ps = std::make_shared<ParamSet>();
+    if (!gen_pass(&a, R, sizeof(V) == 16, hm, ps->jp, false)) return nullptr;
+    ps->key = plan_key(a, R, sizeof(V), ps->jp.classes);
+    ps->memo = get_memo(ps->key);
+    if (!ps->memo) {
+        auto m = std::make_shared<JitMemo>();
+        JitPass full;
+        if (!gen_pass(&a, R, sizeof(V) == 16, hm, full, true)) return nullptr;
+        m->src.swap(full.src);
+        ps->memo = put_memo(ps->key, m);
+    }
+    if (!a.batched) {
+        ps->values = values;
+        std::lock_guard<std::mutex> lock(L.mu);
+        if (L.sets.size() >= kParamSets) L.sets.erase(L.sets.begin());
+        else g_plan_bytes += values.size() + 8 * ps->jp.params.size();
+        L.sets.push_back(ps);
+    }
+    return ps;
+}
+
 // Launch the run-time compiled kernel of a planned register pass, if the
 // compiler has it ready (mode SYNC: after compiling it); returns 1 when it
 // was launched, 0 when the generic kernel has to run, < 0 on error.
 template <typename V>
-int launch_jit(V* vec, const RegArgs& args, int R, const V* hm, const V* mats, double* partials, cudaStream_t st) {
+int launch_jit(V* vec, PlanLaunch& L, int R, const V* hm, const V* mats, double* partials, cudaStream_t st) {
     const int jm = jit::mode();
     if (jm == QS_JIT_OFF || hm == nullptr) return 0;
-    static thread_local JitPass jp;
-    if (!gen_pass(&args, R, sizeof(V) == 16, hm, jp, false)) return 0;
-    // during stream capture nothing is compiled or loaded: a kernel that is
-    // not loaded yet on this device leaves the pass to the generic kernel
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusActive;
-    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    const std::shared_ptr<const ParamSet> ps = get_params<V>(L, R, hm);
+    if (!ps) return 0;
+    const JitPass& jp = ps->jp;
+    const RegArgs& args = L.args;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    static std::mutex memo_mu;
-    static std::unordered_map<uint64_t, std::shared_ptr<JitMemo>> memo;
-    const uint64_t key = plan_key(args, R, sizeof(V), jp.classes);
-    std::shared_ptr<JitMemo> m;
+    JitMemo& m = *ps->memo;
+    void* fn = nullptr;
+    int occ = 0;
+    std::string src;
     {
-        std::lock_guard<std::mutex> lock(memo_mu);
-        auto it = memo.find(key);
-        if (it != memo.end()) m = it->second;
+        std::lock_guard<std::mutex> lock(memo_mu());
+        fn = m.fn[dev];
+        occ = m.occ[dev];
+        if (fn == nullptr) src = m.src;
     }
-    void* fn = m ? m->fn[dev] : nullptr;
-    int occ = m ? m->occ[dev] : 0;
     if (fn == nullptr) {
-        if (!m) {
-            m = std::make_shared<JitMemo>();
+        // during stream capture nothing is compiled or loaded: a kernel that is
+        // not loaded yet on this device leaves the pass to the generic kernel
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusActive;
+        const bool capturing = cs != cudaStreamCaptureStatusNone;
+        if (src.empty()) {  // loaded on another device only: regenerate the text
             JitPass full;
             if (!gen_pass(&args, R, sizeof(V) == 16, hm, full, true)) return 0;
-            m->src.swap(full.src);
-            std::lock_guard<std::mutex> lock(memo_mu);
-            if (memo.size() > 4096) memo.clear();  // bounded: plans are cheap to regenerate
-            memo[key] = m;
+            src.swap(full.src);
         }
-        if (m->src.empty()) {  // loaded on another device only: regenerate the text
-            JitPass full;
-            if (!gen_pass(&args, R, sizeof(V) == 16, hm, full, true)) return 0;
-            m->src.swap(full.src);
-        }
-        fn = jit::lookup(m->src, "qs_pass", jm == QS_JIT_SYNC && !capturing, !capturing, jp.threads, jp.smem, &occ);
+        fn = jit::lookup(src, "qs_pass", jm == QS_JIT_SYNC && !capturing, !capturing, jp.threads, jp.smem, &occ);
         if (fn != nullptr) {
-            std::lock_guard<std::mutex> lock(memo_mu);
-            m->fn[dev] = fn;
-            m->occ[dev] = occ;
-            std::string().swap(m->src);
+            std::lock_guard<std::mutex> lock(memo_mu());
+            m.fn[dev] = fn;
+            m.occ[dev] = occ;
+            std::string().swap(m.src);
         }
     }
     if (fn == nullptr) {
@@ -422,7 +562,7 @@ int launch_jit(V* vec, const RegArgs& args, int R, const V* hm, const V* mats, d
     void* vp = vec;
     const void* mp = mats;
     void* pp = partials;
-    void* params[] = {&vp, jp.params.data(), &mp, &pp};
+    void* params[] = {&vp, const_cast<uint64_t*>(jp.params.data()), &mp, &pp};
     rc = jit::launch(fn, unsigned(ntiles < cap ? ntiles : cap), unsigned(jp.threads), jp.smem, st, params);
     if (rc) return rc;
     jit::count_launch(true);
@@ -443,35 +583,38 @@ inline int jit_reg_bits(int generic_r) {
 template <typename V, int R, bool EXP, bool BIG>
 int launch_reg_k(V* vec, int n, const qs_pass& ps, const qs_op* ops, const V* mats, double* partials, cudaStream_t st,
                  const V* hm = nullptr) {
-    static thread_local RegArgs args;
-    config_smem((const void*)k_fused_reg<V, R, EXP, BIG>);
-    std::vector<int> rem(ps.op_count);
-    for (int i = 0; i < ps.op_count; ++i) rem[i] = i;
     const int nb = sizeof(V) == 16 ? 3 : 4;  // bank-group bits of a shared-memory phase
     const int RJ = jit_reg_bits(R);
-    while (!rem.empty()) {
-        const int next = ps.op_begin + rem.front();
-        if (!EXP && RJ != R && ps.k - RJ >= 5 && ps.k - RJ <= 8) {
-            // a generated pass with its own register width plans its own launch;
-            // the generic kernel re-plans the same ops when it is not ready
-            std::vector<int> saved = rem;
-            if (build_reg(ps, ops, rem, n, RJ, nb, args) > 0) {
-                int jr = launch_jit<V>(vec, args, RJ, hm, mats, partials, st);
+    qs_pass rest = ps;
+    std::vector<qs_op> rest_ops;
+    if (!EXP && RJ != R && ps.k - RJ >= 5 && ps.k - RJ <= 8) {
+        // a generated pass with its own register width has its own plan; from
+        // the first launch that is not ready on, the generic kernel's plan of
+        // the remaining ops takes over
+        if (const std::shared_ptr<PassPlan> plan = get_plan(ps, ops, n, RJ, nb)) {
+            size_t done = 0;
+            for (; done < plan->launches.size(); ++done) {
+                const int jr = launch_jit<V>(vec, *plan->launches[done], RJ, hm, mats, partials, st);
                 if (jr < 0) return jr;
-                if (jr == 1) continue;
+                if (jr == 0) break;
             }
-            rem.swap(saved);
+            if (done == plan->launches.size()) return QS_OK;
+            for (int i : plan->launches[done]->rem) rest_ops.push_back(ops[ps.op_begin + i]);
+            rest.op_begin = 0;
+            rest.op_count = int(rest_ops.size());
+            ops = rest_ops.data();
         }
-        int used = build_reg(ps, ops, rem, n, R, nb, args);
-        if (used <= 0) {
-            set_error("qs_apply_fused: op %d does not fit a register tile", next);
-            return QS_EINVAL;
-        }
+    }
+    const std::shared_ptr<PassPlan> plan = get_plan(rest, ops, n, R, nb);
+    if (!plan) return QS_EINVAL;
+    for (const auto& L : plan->launches) {
+        const RegArgs& args = L->args;
         if (EXP || RJ == R) {
-            int jr = launch_jit<V>(vec, args, R, hm, mats, partials, st);
+            const int jr = launch_jit<V>(vec, *L, R, hm, mats, partials, st);
             if (jr < 0) return jr;
             if (jr == 1) continue;
         }
+        config_smem((const void*)k_fused_reg<V, R, EXP, BIG>);
         const int threads = 1 << (ps.k - R);
         const size_t smem = reg_smem_bytes<V>(args, R, EXP);
         if (smem > size_t(smem_optin())) {

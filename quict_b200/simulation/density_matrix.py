@@ -23,7 +23,7 @@ import numpy as np
 import torch
 
 from .. import _native as N
-from .engine import Engine, require_cuda
+from .engine import Engine, KeyedOps, require_cuda
 from .fusion import _full_matrix
 from .lowering import Op, classify, lower_gate
 from .state_vector import StateArray
@@ -173,6 +173,7 @@ class DensityMatrixSimulator:
             if any(op.kind in ("measure", "reset", "perm") for op in ops):
                 ops = None
             else:
+                ops = KeyedOps(ops)
                 self._lowered[key] = (noise_model, self._circuit, ops)  # holds the model: its id stays unique
                 while len(self._lowered) > 8:
                     self._lowered.pop(next(iter(self._lowered)))

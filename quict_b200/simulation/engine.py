@@ -67,6 +67,41 @@ class _Program:
         flush()
 
 
+class _Content:
+    """Contents of an op sequence as a dictionary key, hashed once."""
+    __slots__ = ("parts", "_hash")
+
+    def __init__(self, parts: tuple):
+        self.parts, self._hash = parts, hash(parts)
+
+    def __hash__(self):
+        return self._hash
+
+    def __eq__(self, other):
+        return self is other or (isinstance(other, _Content) and self.parts == other.parts)
+
+
+def _content_key(ops: Sequence[Op]) -> Optional[_Content]:
+    parts = []
+    for op in ops:
+        if op.batch is not None or op.tag is not None or op.kind not in ("mat", "diag", "antidiag", "swap"):
+            return None
+        parts.append((op.kind, op.tbits, op.cbits, op.mat.tobytes()))
+    return _Content(tuple(parts))
+
+
+class KeyedOps(tuple):
+    """Lowered ops that a simulator keeps for a circuit, with their content
+    key (a replayed circuit does not read every matrix again)."""
+
+    @property
+    def content(self) -> Optional[_Content]:
+        c = self.__dict__.get("_content", False)
+        if c is False:
+            c = self.__dict__["_content"] = _content_key(self)
+        return c
+
+
 class Workspace:
     """Grow-only device scratch owned by torch; handed to libqsim as (ptr, bytes)."""
 
@@ -239,12 +274,8 @@ class Engine:
         """Exact key of an op sequence (None: not kept, e.g. batched or tagged ops)."""
         if not ops:
             return None
-        parts = [n, str(vec.dtype), self.knobs(vec, n)]
-        for op in ops:
-            if op.batch is not None or op.tag is not None or op.kind not in ("mat", "diag", "antidiag", "swap"):
-                return None
-            parts.append((op.kind, op.tbits, op.cbits, op.mat.tobytes()))
-        return tuple(parts)
+        content = ops.content if isinstance(ops, KeyedOps) else _content_key(ops)
+        return None if content is None else (n, vec.dtype, self.knobs(vec, n), content)
 
     def _run_program(self, vec: torch.Tensor, n: int, prog: "_Program"):
         st = self.stream

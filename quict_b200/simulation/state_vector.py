@@ -15,7 +15,7 @@ import numpy as np
 import torch
 
 from .. import _native as N
-from .engine import Engine, require_cuda
+from .engine import Engine, KeyedOps, require_cuda
 from .lowering import Op, lower_gate
 
 
@@ -177,7 +177,7 @@ class StateVectorSimulator:
                 if any(op.kind in ("measure", "reset", "perm") for op in ops):
                     ops = None
                 else:
-                    self._lowered[key] = ops
+                    ops = self._lowered[key] = KeyedOps(ops)
                     while len(self._lowered) > 8:
                         self._lowered.pop(next(iter(self._lowered)))
             if ops is not None:
@@ -333,16 +333,23 @@ def _circuit_key(gates, n: int, legacy: bool):
     parts = [n, legacy]
     for g in gates:
         t = getattr(g, "type", None)
-        name = getattr(t, "name", None)
-        if name is None or name in ("measure", "reset") or _is_trigger(g):
+        # an Enum member's plain attribute first: its `name` is a Python-level property
+        name = getattr(t, "_name_", None) or getattr(t, "name", None)
+        if name is None or name == "measure" or name == "reset":
             return None
-        k = (name, tuple(g.cargs), tuple(g.targs), tuple(g.pargs), str(getattr(g, "precision", "")))
-        if name not in _PARAM_DETERMINED:
+        if not hasattr(type(g), "matrix_type") and _is_trigger(g):
+            return None
+        prec = getattr(g, "precision", "")
+        if not isinstance(prec, (type, str)):
+            prec = str(prec)
+        c, q = g.cargs, g.targs
+        if name in _PARAM_DETERMINED:
+            parts.append((name, prec, len(c), len(q), *c, *q, *g.pargs))
+        else:
             m = g.matrix
             if m is None:
                 return None
-            k = k + (np.asarray(m).tobytes(),)
-        parts.append(k)
+            parts.append((name, prec, len(c), len(q), *c, *q, *g.pargs, np.asarray(m).tobytes()))
     return tuple(parts)
 
 
