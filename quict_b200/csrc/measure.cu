@@ -3,8 +3,8 @@
 // Sampling replaces the reference's shots x qubits loop (one reduction, one
 // device->host read and one collapse kernel per qubit per shot,
 // statevector_simulator.py:595-626) with a sum tree built once: FP64 sums of
-// 2^B-amplitude blocks at the leaves, a binary heap above them.  Each shot is
-// one warp that walks the heap from the root (qubit 0 = the vector's top bit
+// 2^B-amplitude blocks at the leaves, a binary tree above them.  Each shot is
+// one warp that walks the tree from the root (qubit 0 = the vector's top bit
 // first) and finishes inside its leaf block from the block's own amplitudes.
 #include <mutex>
 
@@ -15,7 +15,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kReduceCtas = 1024;     // partial-sum slots in the reduce workspace
-constexpr int kBlockBits = 10;        // leaf block = 2^10 probabilities
 
 // p_i of a probability source
 template <typename V, int SRC>
@@ -47,12 +46,27 @@ __device__ __forceinline__ double block_sum(double x) {
 }
 
 // Sum of p over the compact space with `bit` removed (bit < 0: everything).
+// Eight loads in flight per thread: 25 qubits in complex64 (B200), half of
+// the 256 MB: 33 us (51 us on the lowest bits, where every sector is read),
+// 62-73 us with one.
 template <typename V, int SRC>
 __global__ void __launch_bounds__(kThreads)
 k_partial(const V* __restrict__ s, uint64_t items, int bit, uint64_t dstride, double* __restrict__ part) {
+    constexpr int U = 8;
     double acc = 0.0;
     const uint64_t stride = uint64_t(gridDim.x) * kThreads;
-    for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < items; j += stride) {
+    uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x;
+    for (; j + (U - 1) * stride < items; j += U * stride) {
+        V v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t q = j + u * stride, i = bit >= 0 ? insert0(q, bit) : q;
+            v[u] = s[SRC == QS_SRC_SV ? i : i * dstride];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc += SRC == QS_SRC_SV ? cnorm2(v[u]) : double(v[u].x);
+    }
+    for (; j < items; j += stride) {
         uint64_t i = bit >= 0 ? insert0(j, bit) : j;
         acc += prob_at<V, SRC>(s, i, dstride);
     }
@@ -67,62 +81,165 @@ __global__ void __launch_bounds__(kThreads) k_finish(const double* __restrict__ 
     if (threadIdx.x == 0) *out = acc;
 }
 
+// Both walk the pairs of `bit`, four in flight per thread, and read only the
+// half that is kept: 25 qubits in complex64 (B200), 256 MB: collapse 65-88 us
+// (65-95 us when every amplitude was visited one at a time), reset 67 us (131
+// us with a division per component).
 template <typename V>
-__global__ void __launch_bounds__(kThreads) k_collapse(V* __restrict__ v, uint64_t N, int bit, int outcome, double scale) {
-    const uint64_t stride = uint64_t(gridDim.x) * kThreads;
-    for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < N; i += stride) {
-        if (int((i >> bit) & 1) == outcome) {
-            V a = v[i];
-            a.x *= scale; a.y *= scale;
-            v[i] = a;
-        } else {
-            v[i] = mk<V>(0.0, 0.0);
+__global__ void __launch_bounds__(kThreads) k_collapse(V* __restrict__ v, uint64_t items, int bit, int outcome, double scale) {
+    constexpr int U = 4;
+    const uint64_t stride = uint64_t(gridDim.x) * kThreads, off = uint64_t(1) << bit;
+    const uint64_t keep = outcome ? off : 0;
+    for (uint64_t j0 = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j0 < items; j0 += U * stride) {
+        V a[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (j0 + u * stride < items) a[u] = v[insert0(j0 + u * stride, bit) | keep];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 + u * stride >= items) continue;
+            const uint64_t i0 = insert0(j0 + u * stride, bit);
+            a[u].x *= scale; a[u].y *= scale;
+            v[i0 | keep] = a[u];
+            v[i0 | (keep ^ off)] = mk<V>(0.0, 0.0);
         }
     }
+}
+
+// x / alpha for a given r = 1 / alpha: one correction step on x r gives the
+// correctly rounded quotient (Markstein, IBM J. Res. Dev. 34(1), 1990).  A
+// quotient of a component that is not finite or too small for the remainder
+// to be exact is divided.
+__device__ __forceinline__ double div_by(double x, double alpha, double r) {
+    const double q = x * r;
+    if (!(fabs(q) > 1e-280 && fabs(q) < 1e300)) return x / alpha;
+    return fma(fma(-q, alpha, x), r, q);
+}
+__device__ __forceinline__ float div_by(float x, double alpha, double r) {
+    return float(double(x) * r);  // within half a unit of the float result either way
 }
 
 // Reference reset rule: alpha = sqrt(P0); alpha < 1e-6 -> v0 <- v1, else
 // v0 <- v0 / alpha; v1 <- 0 either way.
 template <typename V>
 __global__ void __launch_bounds__(kThreads) k_reset(V* __restrict__ v, uint64_t items, int bit, double alpha, bool move) {
-    const uint64_t stride = uint64_t(gridDim.x) * kThreads;
-    const uint64_t off = uint64_t(1) << bit;
-    for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < items; j += stride) {
-        uint64_t i0 = insert0(j, bit);
-        V a;
-        if (move) {
-            a = v[i0 + off];
-        } else {
-            a = v[i0];
-            a.x /= alpha; a.y /= alpha;
+    constexpr int U = 4;
+    const uint64_t stride = uint64_t(gridDim.x) * kThreads, off = uint64_t(1) << bit;
+    const double r = 1.0 / alpha;
+    for (uint64_t j0 = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j0 < items; j0 += U * stride) {
+        V a[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (j0 + u * stride < items) a[u] = v[insert0(j0 + u * stride, bit) | (move ? off : 0)];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 + u * stride >= items) continue;
+            const uint64_t i0 = insert0(j0 + u * stride, bit);
+            if (!move) {
+                a[u].x = div_by(a[u].x, alpha, r);
+                a[u].y = div_by(a[u].y, alpha, r);
+            }
+            v[i0] = a[u];
+            v[i0 | off] = mk<V>(0.0, 0.0);
         }
-        v[i0] = a;
-        v[i0 + off] = mk<V>(0.0, 0.0);
     }
 }
 
 // -------------------------------------------------------------- sum tree
-// ws layout: double tree[2 * nleaf]; heap with root at 1, leaves at
-// [nleaf, 2*nleaf), leaf b = sum of p over block b (2^bb probabilities).
+// FP64 sums of leaf blocks of 2^bb probabilities, and above them every fifth
+// level of the binary tree: level 0 holds the leaves, an entry of level j + 1
+// sums 32 entries of level j (the top one fewer), the last level is the total.
+// The four levels in between are never stored: a warp that holds the 32
+// entries below a node has them from five butterfly steps, so a shot costs
+// one coalesced load per five levels instead of a dependent load per level.
+// 26 qubits in complex64, 100,000 shots (B200): a heap with every level stored,
+// one dependent load per level and 32 elements per lane in the leaf took
+// 649 us + 23 us for 16 launches of single levels; this takes 153 + 6 us, and
+// the leaves 75 us (120 us with one load in flight).  What is left is the
+// leaves' 8 KB a shot.
+constexpr int kMaxLevels = 8;  // 30 tree bits over the leaves, five per level, and the root
+
+struct TreeShape {
+    int bb, levels;             // leaf bits; stored levels
+    int lg[kMaxLevels];         // log2 of a level's entries
+    uint64_t off[kMaxLevels];   // its first entry
+    uint64_t total;             // entries of all levels
+};
+
+constexpr int kBlockBits = 10;  // leaf block = 2^10 probabilities: 32 rows of 32
+
+TreeShape tree_shape(int n) {
+    TreeShape t{};
+    t.bb = n < kBlockBits ? n : kBlockBits;
+    int lg = n - t.bb;
+    for (;;) {
+        t.lg[t.levels] = lg;
+        t.off[t.levels++] = t.total;
+        t.total += uint64_t(1) << lg;
+        if (lg == 0) break;
+        lg = lg > 5 ? lg - 5 : 0;
+    }
+    return t;
+}
+
+// Sum over the warp, lanes paired by ascending distance (the order in which
+// the descent recomputes the levels between two stored ones).
+__device__ __forceinline__ double tree_sum(double x) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// One warp per leaf, eight loads in flight per lane.
 template <typename V, int SRC>
 __global__ void __launch_bounds__(kThreads)
-k_leaves(const V* __restrict__ s, uint64_t nleaf, int bb, uint64_t dstride, double* __restrict__ tree) {
+k_leaves(const V* __restrict__ s, int bb, uint64_t nleaf, uint64_t dstride, double* __restrict__ leaf) {
+    constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const uint64_t warps = uint64_t(gridDim.x) * (kThreads / 32);
-    const uint64_t bsz = uint64_t(1) << bb;
     for (uint64_t b = uint64_t(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); b < nleaf; b += warps) {
+        const uint64_t base = (b << bb) + lane;
         double acc = 0.0;
-        for (uint64_t e = lane; e < bsz; e += 32) acc += prob_at<V, SRC>(s, b * bsz + e, dstride);
-        acc = warp_sum(acc);
-        if (lane == 0) tree[nleaf + b] = acc;
+        if (bb == kBlockBits) {
+            for (int r = 0; r < 32; r += U) {
+                V v[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) v[i] = s[(base + 32 * (r + i)) * (SRC == QS_SRC_SV ? 1 : dstride)];
+#pragma unroll
+                for (int i = 0; i < U; ++i) acc += SRC == QS_SRC_SV ? cnorm2(v[i]) : double(v[i].x);
+            }
+        } else {
+            for (int e = lane; e < (1 << bb); e += 32) acc += prob_at<V, SRC>(s, base - lane + e, dstride);
+        }
+        acc = tree_sum(acc);
+        if (lane == 0) leaf[b] = acc;
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_level(double* __restrict__ tree, uint64_t lo, uint64_t cnt) {
-    const uint64_t stride = uint64_t(gridDim.x) * kThreads;
-    for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < cnt; j += stride) {
-        uint64_t i = lo + j;
-        tree[i] = tree[2 * i] + tree[2 * i + 1];
+// One warp per entry of the level above `in` (2^lg entries).
+__global__ void __launch_bounds__(kThreads) k_level(const double* __restrict__ in, int lg, double* __restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t warps = uint64_t(gridDim.x) * (kThreads / 32);
+    const uint64_t cnt = lg > 5 ? uint64_t(1) << (lg - 5) : 1;
+    const uint64_t size = uint64_t(1) << lg;
+    for (uint64_t g = uint64_t(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); g < cnt; g += warps) {
+        const double t = tree_sum(32 * g + lane < size ? in[32 * g + lane] : 0.0);
+        if (lane == 0) out[g] = t;
+    }
+}
+
+// All levels above `from`, in one block (from at most 2^14 entries): no launch
+// between two small levels.
+__global__ void __launch_bounds__(1024) k_top(double* __restrict__ tree, const __grid_constant__ TreeShape t, int from) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int j = from; j + 1 < t.levels; ++j) {
+        const double* in = tree + t.off[j];
+        const uint64_t size = uint64_t(1) << t.lg[j], cnt = uint64_t(1) << t.lg[j + 1];
+        for (uint64_t g = w; g < cnt; g += 32) {
+            const double x = tree_sum(32 * g + lane < size ? in[32 * g + lane] : 0.0);
+            if (lane == 0) tree[t.off[j + 1] + g] = x;
+        }
+        __syncthreads();
     }
 }
 
@@ -137,85 +254,95 @@ __device__ __forceinline__ bool cdf_right(double uc, double acc, double sl, doub
     return !(uc <= acc + sl);
 }
 
-// One warp per shot.  Within the leaf block lane l owns elements
-// [l*E, (l+1)*E), E = 2^bb / 32 (or one element per lane for tiny blocks).
+// A shot's position in the decision sequence: the uniform in use and, in CDF
+// mode, the mass strictly left of the current node.
+struct Draw {
+    const double* us;
+    int lvl, n;
+    double uc, acc;
+};
+
+// Walk down nb <= 5 levels below a node whose 2^nb entries are the lanes' x;
+// returns the lane of the entry reached.
+template <int MODE>
+__device__ __forceinline__ int descend(double x, int nb, Draw& d) {
+    double t[6];
+    t[0] = x;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) t[k + 1] = t[k] + __shfl_xor_sync(0xffffffffu, t[k], 1 << k);
+    int lo = 0;
+#pragma unroll
+    for (int k = 4; k >= 0; --k) {
+        if (k >= nb) continue;  // warp-uniform
+        const double sl = __shfl_sync(0xffffffffu, t[k], lo), sr = __shfl_sync(0xffffffffu, t[k], lo + (1 << k));
+        bool right;
+        if (MODE == QS_SAMPLE_SEQ) {
+            right = d.uc > sl / (sl + sr);
+            ++d.lvl;
+            d.uc = d.us[d.lvl < d.n ? d.lvl : d.n - 1];
+        } else {
+            right = cdf_right(d.uc, d.acc, sl, sr);
+            if (right) d.acc += sl;
+        }
+        if (right) lo += 1 << k;
+    }
+    return lo;
+}
+
+// One warp per shot: through the stored levels, then the leaf block's rows of
+// 32, then the row.
 template <typename V, int SRC, int MODE>
 __global__ void __launch_bounds__(kThreads)
-k_sample(const V* __restrict__ s, int n, uint64_t nleaf, int bb, uint64_t dstride, const double* __restrict__ tree,
+k_sample(const V* __restrict__ s, int n, const __grid_constant__ TreeShape t, uint64_t dstride, const double* __restrict__ tree,
          const double* __restrict__ u, int64_t shots, int64_t* __restrict__ out) {
-    constexpr int EMAX = (1 << kBlockBits) / 32;
     const int lane = threadIdx.x & 31;
     const int64_t warps = int64_t(gridDim.x) * (kThreads / 32);
-    const int top = n - bb;  // heap levels above the leaves
-    const int bsz = 1 << bb;
-    const int E = bsz >= 32 ? bsz / 32 : 1;
+    const int rowbits = t.bb > 5 ? t.bb - 5 : 0, lanebits = t.bb - rowbits;
     for (int64_t shot = int64_t(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5); shot < shots; shot += warps) {
-        const double* us = MODE == QS_SAMPLE_SEQ ? u + shot * n : u + shot;
+        Draw d;
+        d.us = MODE == QS_SAMPLE_SEQ ? u + shot * n : u + shot;
+        d.lvl = 0;
+        d.n = n;
+        d.acc = 0.0;
         // CDF mode compares against unnormalised FP64 partial sums, so the
         // uniform is scaled by the total mass (the root): a state whose norm
         // has drifted below 1 (complex64, a density matrix's trace) then
         // never runs off the end of the distribution
-        double uc = MODE == QS_SAMPLE_SEQ ? us[0] : us[0] * tree[1];
-        double acc = 0.0;  // CDF mode: mass strictly left of the current node
-        uint64_t node = 1;
-        for (int lvl = 0; lvl < top; ++lvl) {
-            double sl = tree[2 * node], sr = tree[2 * node + 1];
-            bool right;
-            if (MODE == QS_SAMPLE_SEQ) {
-                double tot = sl + sr;
-                right = uc > sl / tot;
-                uc = us[lvl + 1 < n ? lvl + 1 : n - 1];
-            } else {
-                right = cdf_right(uc, acc, sl, sr);
-                if (right) acc += sl;
-            }
-            node = 2 * node + (right ? 1 : 0);
+        d.uc = MODE == QS_SAMPLE_SEQ ? d.us[0] : d.us[0] * tree[t.off[t.levels - 1]];
+        uint64_t node = 0;
+        for (int j = t.levels - 2; j >= 0; --j) {
+            const int nb = t.lg[j] - t.lg[j + 1];
+            const double x = lane < (1 << nb) ? tree[t.off[j] + (node << nb) + lane] : 0.0;
+            node = (node << nb) + descend<MODE>(x, nb, d);
         }
-        const uint64_t blk = node - nleaf;
-        const uint64_t base = blk * uint64_t(bsz);
-        double p[EMAX];
+        uint64_t base = node << t.bb;
+        if (rowbits == 5) {
+            // the 32 rows' sums, lane r ending up with row r: five exchanges in
+            // which each half of the lanes keeps half of the rows
+            double p[32];
 #pragma unroll
-        for (int e = 0; e < EMAX; ++e) {
-            int idx = lane * E + e;
-            p[e] = (e < E && idx < bsz) ? prob_at<V, SRC>(s, base + idx, dstride) : 0.0;
-        }
-        // descend inside the block over ranges [lo, lo + size)
-        int lo = 0;
-        int lvl = top;
-        for (int size = bsz; size > 1; size >>= 1, ++lvl) {
-            const int half = size >> 1;
-            double sl, sr;
-            if (half >= E) {
-                // whole lanes: lanes [lo/E, (lo+half)/E) left, [(lo+half)/E, (lo+size)/E) right
-                double mine = 0.0;
+            for (int r = 0; r < 32; ++r) p[r] = prob_at<V, SRC>(s, base + 32 * r + lane, dstride);
 #pragma unroll
-                for (int e = 0; e < EMAX; ++e) mine += (e < E) ? p[e] : 0.0;
-                const int l0 = lo / E, lm = (lo + half) / E, l1 = (lo + size) / E;
-                sl = warp_sum((lane >= l0 && lane < lm) ? mine : 0.0);
-                sr = warp_sum((lane >= lm && lane < l1) ? mine : 0.0);
-            } else {
-                // inside one lane
-                const int owner = lo / E, off = lo % E;
-                double a = 0.0, b = 0.0;
+            for (int h = 16; h > 0; h >>= 1) {
+                const bool upper = lane & h;
 #pragma unroll
-                for (int e = 0; e < EMAX; ++e) {
-                    if (e >= off && e < off + half) a += p[e];
-                    if (e >= off + half && e < off + size) b += p[e];
+                for (int i = 0; i < h; ++i) {
+                    const double give = upper ? p[i] : p[i + h], keep = upper ? p[i + h] : p[i];
+                    p[i] = keep + __shfl_xor_sync(0xffffffffu, give, h);
                 }
-                sl = __shfl_sync(0xffffffffu, a, owner);
-                sr = __shfl_sync(0xffffffffu, b, owner);
             }
-            bool right;
-            if (MODE == QS_SAMPLE_SEQ) {
-                right = uc > sl / (sl + sr);
-                uc = us[lvl + 1 < n ? lvl + 1 : n - 1];
-            } else {
-                right = cdf_right(uc, acc, sl, sr);
-                if (right) acc += sl;
+            base += 32 * uint64_t(descend<MODE>(p[0], 5, d));
+        } else if (rowbits > 0) {
+            double rows = 0.0;
+            for (int r = 0; r < (1 << rowbits); ++r) {
+                const double x = tree_sum(prob_at<V, SRC>(s, base + 32 * r + lane, dstride));
+                if (lane == r) rows = x;
             }
-            if (right) lo += half;
+            base += 32 * uint64_t(descend<MODE>(rows, rowbits, d));
         }
-        if (lane == 0) out[shot] = int64_t(base + lo);
+        const double p = lane < (1 << lanebits) ? prob_at<V, SRC>(s, base + lane, dstride) : 0.0;
+        base += descend<MODE>(p, lanebits, d);
+        if (lane == 0) out[shot] = int64_t(base);
     }
 }
 
@@ -250,37 +377,33 @@ int reduce_t(const void* src, int n, int src_kind, int bit, void* ws, double* ou
     return QS_OK;
 }
 
-int tree_shape(int n, uint64_t* nleaf, int* bb) {
-    *bb = n < kBlockBits ? n : kBlockBits;
-    *nleaf = uint64_t(1) << (n - *bb);
-    return QS_OK;
-}
-
 template <typename V>
 int prepare_t(const void* src, int n, int src_kind, double* tree, cudaStream_t st) {
     const V* s = static_cast<const V*>(src);
-    uint64_t nleaf; int bb;
-    tree_shape(n, &nleaf, &bb);
-    uint64_t dstride = (uint64_t(1) << n) + 1;
-    unsigned grid = grid_for(nleaf, kThreads / 32, 8, 4);
-    if (src_kind == QS_SRC_SV) k_leaves<V, QS_SRC_SV><<<grid, kThreads, 0, st>>>(s, nleaf, bb, dstride, tree);
-    else                       k_leaves<V, QS_SRC_DM><<<grid, kThreads, 0, st>>>(s, nleaf, bb, dstride, tree);
-    for (uint64_t lo = nleaf / 2; lo >= 1; lo /= 2)
-        k_level<<<grid_for(lo, kThreads, 8), kThreads, 0, st>>>(tree, lo, lo);
+    const TreeShape t = tree_shape(n);
+    const uint64_t nleaf = uint64_t(1) << t.lg[0];
+    const uint64_t dstride = (uint64_t(1) << n) + 1;
+    const unsigned grid = grid_for(nleaf, kThreads / 32, 8, 4);
+    if (src_kind == QS_SRC_SV) k_leaves<V, QS_SRC_SV><<<grid, kThreads, 0, st>>>(s, t.bb, nleaf, dstride, tree);
+    else                       k_leaves<V, QS_SRC_DM><<<grid, kThreads, 0, st>>>(s, t.bb, nleaf, dstride, tree);
+    int j = 0;
+    for (; j + 1 < t.levels && t.lg[j] > 14; ++j)  // levels that one block would take long over
+        k_level<<<grid_for(uint64_t(1) << t.lg[j + 1], kThreads / 32, 8), kThreads, 0, st>>>(tree + t.off[j], t.lg[j],
+                                                                                            tree + t.off[j + 1]);
+    if (j + 1 < t.levels) k_top<<<1, 1024, 0, st>>>(tree, t, j);
     QS_CHECK_LAUNCH("qs_sample_prepare");
     return QS_OK;
 }
 
 template <typename V>
-int sample_t(const void* src, int n, int src_kind, const double* tree, const double* u, int64_t shots, int mode,
-             int64_t* out, cudaStream_t st) {
+int sample_t(const void* src, int n, int src_kind, const double* tree, const double* u, int64_t shots,
+             int mode, int64_t* out, cudaStream_t st) {
     const V* s = static_cast<const V*>(src);
-    uint64_t nleaf; int bb;
-    tree_shape(n, &nleaf, &bb);
+    const TreeShape t = tree_shape(n);
     uint64_t dstride = (uint64_t(1) << n) + 1;
     unsigned grid = grid_for(uint64_t(shots), kThreads / 32, 8, 4);
 #define QS_SAMPLE_LAUNCH(SRC, MODE) \
-    k_sample<V, SRC, MODE><<<grid, kThreads, 0, st>>>(s, n, nleaf, bb, dstride, tree, u, shots, out)
+    k_sample<V, SRC, MODE><<<grid, kThreads, 0, st>>>(s, n, t, dstride, tree, u, shots, out)
     if (src_kind == QS_SRC_SV) {
         if (mode == QS_SAMPLE_SEQ) QS_SAMPLE_LAUNCH(QS_SRC_SV, QS_SAMPLE_SEQ);
         else                       QS_SAMPLE_LAUNCH(QS_SRC_SV, QS_SAMPLE_CDF);
@@ -332,10 +455,10 @@ extern "C" int qs_collapse(void* vec, int n, int dtype, int bit, int outcome, do
     if (rc) return rc;
     QS_REQUIRE(bit >= 0 && bit < n, "bit %d outside [0, %d)", bit, n);
     QS_REQUIRE(outcome == 0 || outcome == 1, "outcome must be 0 or 1");
-    uint64_t N = uint64_t(1) << n;
-    unsigned grid = grid_for(N, kThreads * 4, 8);
-    if (dtype == QS_C128) k_collapse<double2><<<grid, kThreads, 0, as_stream(stream)>>>((double2*)vec, N, bit, outcome, scale);
-    else                  k_collapse<float2><<<grid, kThreads, 0, as_stream(stream)>>>((float2*)vec, N, bit, outcome, scale);
+    uint64_t items = uint64_t(1) << (n - 1);
+    unsigned grid = grid_for(items, kThreads * 4, 8);
+    if (dtype == QS_C128) k_collapse<double2><<<grid, kThreads, 0, as_stream(stream)>>>((double2*)vec, items, bit, outcome, scale);
+    else                  k_collapse<float2><<<grid, kThreads, 0, as_stream(stream)>>>((float2*)vec, items, bit, outcome, scale);
     QS_CHECK_LAUNCH("qs_collapse");
     return QS_OK;
 }
@@ -355,9 +478,8 @@ extern "C" int qs_reset(void* vec, int n, int dtype, int bit, double p0, void* s
 }
 
 extern "C" size_t qs_sample_ws_bytes(int n) {
-    uint64_t nleaf; int bb;
-    tree_shape(n, &nleaf, &bb);
-    return sizeof(double) * 2 * nleaf;
+    const int bb = n < kBlockBits ? n : kBlockBits;
+    return sizeof(double) * (size_t(2) << (n - bb));  // the levels take half of it and a bit
 }
 
 extern "C" int qs_sample_prepare(const void* src, int n, int dtype, int src_kind, void* ws, size_t ws_bytes,
