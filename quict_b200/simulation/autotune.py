@@ -55,9 +55,30 @@ class Knobs:
                      math.inf if c is None else float(c))
 
 
-def default_knobs(esize: int) -> Knobs:
-    """Settings used when the cache has no entry (k = 12 / 13, 32-amplitude runs, 2-bit merging)."""
-    return Knobs(12 if esize == 16 else 13, 5, 2)
+def default_knobs(esize: int, n: Optional[int] = None) -> Knobs:
+    """Settings used when the cache has no entry: 32-amplitude runs, 2-bit
+    merging, and a tile width by the size of the state.  200 random gates on
+    uniform qubits (B200, device time):
+
+      complex128, k = 10 / 11 / 12: 14 qubits 27 / 27 / 37 us, 18 qubits 37 / 35 /
+        43 us, 22 qubits 222 / 227 / 265 us, 24 qubits 1243 / 976 / 1104 us, 26
+        qubits 4.07 / 3.68 / 3.82 ms, 28 qubits 19.4 / 16.0 / 15.9 ms
+      complex64, k = 11 / 12 / 13: 14 qubits 31 / 33 / 39 us, 18 qubits 41 / 37 / 41
+        us, 22 qubits 160 / 150 / 162 us, 24 qubits 536 / 552 / 459 us, 26 qubits
+        2.09 / 1.99 / 1.92 ms, 28 qubits 8.36 / 8.33 / 8.08 ms
+
+    On a small state narrow tiles give more SMs a tile; a state that fits the
+    L2 cache is read cheaply, so several CTAs per SM are worth more passes;
+    beyond it every pass saved counts.  Without `n` (and for density matrices,
+    whose 12-qubit noisy runs took 2.97 ms at k = 12 and 3.20 ms at k = 11): the
+    widest tiles."""
+    if n is None:
+        k = 12 if esize == 16 else 13
+    elif esize == 16:
+        k = 11 if n < 27 else 12
+    else:
+        k = 11 if n < 17 else 12 if n < 24 else 13
+    return Knobs(k, 5, 2)
 
 
 def candidates(esize: int, n: int) -> List[Knobs]:

@@ -178,7 +178,7 @@ class Engine:
         kn = self._resolved.get((esize, n))
         if kn is None:
             kn = self.tuner.lookup(tune_key(torch.cuda.get_device_name(self.device), esize, n, self.tune_kind))
-            kn = kn or default_knobs(esize)
+            kn = kn or default_knobs(esize, n if self.tune_kind == "sv" else None)
             self._resolved[(esize, n)] = kn
         return Knobs(self.tile_bits if self.tile_bits is not None else kn.tile_bits,
                      self.low_bits if self.low_bits is not None else kn.low_bits,
