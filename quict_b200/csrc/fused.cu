@@ -377,7 +377,7 @@ uint64_t plan_key(const RegArgs& a, int R, size_t vsize, const std::vector<uint8
         return e && *e ? atoi(e) : 0;
     }();
     h = fnv(h, &target, sizeof(target));
-    const int single = jit_single_buffer(vsize == 16) ? 1 : 0;
+    const int single = jit_single_buffer(vsize == 16, a.batched || a.nexp > 0) ? 1 : 0;
     h = fnv(h, &single, sizeof(single));
     return fnv(h, classes.data(), classes.size());
 }

@@ -26,12 +26,12 @@
 
 namespace qs {
 
-bool jit_single_buffer(bool c128) {
+bool jit_single_buffer(bool c128, bool tables) {
     static const int env = [] {
         const char* e = getenv("QS_JIT_SINGLE_BUFFER");
         return e && (*e == '0' || *e == '1') ? *e - '0' : -1;
     }();
-    return env >= 0 ? env == 1 : c128;
+    return env >= 0 ? env == 1 : c128 || tables;
 }
 
 namespace {
@@ -537,11 +537,14 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
     // stores, and the smaller footprint lets more CTAs share an SM, whose loads
     // and arithmetic overlap.  Measured on the 30-qubit spread circuit (B200),
     // one buffer against two: complex128 k = 11 270 against 284 ms, complex64
-    // k = 12 164.6 against 163.2 ms, k = 11 168.3 against 166.1 ms; so the
-    // default is single for complex128 and double for complex64.  Fetching only
-    // after the stores: complex128 k = 12 276 ms, now 261 ms (k = 10: 272, 269).
+    // k = 12 164.6 against 163.2 ms, k = 11 168.3 against 166.1 ms.  Passes with
+    // per-instance tables and adjoint passes have registers for two CTAs per SM
+    // at any width, where two 64 KB buffers leave room for one: gradients of 256
+    // parameter sets of a 16-qubit ansatz in complex64 6.98 against 10.88 ms.  So
+    // the default is double for plain complex64 passes only.  Fetching only after
+    // the stores: complex128 k = 12 276 ms, now 261 ms (k = 10: 272, 269).
     // QS_JIT_SINGLE_BUFFER=0/1 overrides it.
-    const bool single = devfn == nullptr && jit_single_buffer(C128);
+    const bool single = devfn == nullptr && jit_single_buffer(C128, batched || a.nexp > 0);
     const int nbuf = single ? 1 : 2;
     out.threads = threads;
     out.smem = sizeof(V) * size_t(nbuf) * (size_t(1) << K) + 8 * size_t(hoff_n) +

@@ -16,8 +16,9 @@ struct JitPass {
 };
 
 // Single-buffered generated kernels (see passgen.cu): QS_JIT_SINGLE_BUFFER=0 / 1,
-// else complex128 only.
-bool jit_single_buffer(bool c128);
+// else every pass but plain complex64 ones (tables: per-instance tables or
+// EXPECT ops).
+bool jit_single_buffer(bool c128, bool tables);
 
 // Generate the planned register pass `regargs` (a RegArgs filled by build_reg;
 // the struct has the same layout in every file that includes regtile.cuh).
