@@ -160,14 +160,14 @@ extern "C" int qs_batch_plan(int dtype, const qs_batch_inst* inst, int ninst, co
         grad_doubles += q.nparams;
         b.w_off = int64_t(wts.size());
         for (int64_t k = 0; k < int64_t(q.nparams) * q.nslots; ++k) wts.push_back(weights[q.w_begin + k]);
-        // observable terms, stably sorted by X mask, with i^popc(x & z) folded in
+        // observable terms in pauli_before order, with i^popc(x & z) folded in
         std::vector<int> order(static_cast<size_t>(q.nterms));
         for (int t = 0; t < q.nterms; ++t) {
             const int g = q.term_begin + t;
             QS_REQUIRE((xmask[g] >> q.n) == 0 && (zmask[g] >> q.n) == 0, "instance %d: term %d acts on bits >= n", i, t);
             order[size_t(t)] = g;
         }
-        std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return xmask[a] < xmask[c]; });
+        std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return pauli_before(xmask[a], zmask[a], xmask[c], zmask[c]); });
         for (int g : order) {
             BTerm tm;
             tm.x = xmask[g];

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "pauli.cuh"
 #include "regtile.cuh"
 
 namespace qs {
@@ -29,7 +30,7 @@ struct __align__(16) BInst {
     int64_t grad_off;   // doubles of the gradient output
 };
 
-struct __align__(16) BTerm {  // an instance's terms are sorted (stably) by x
+struct __align__(16) BTerm {  // an instance's terms are in pauli_before order
     uint64_t x, z;
     double cre, cim;  // coefficient times i^popc(x & z)
 };
@@ -84,9 +85,39 @@ __device__ __forceinline__ double2 block_sum(double a, double b) {
     return s;
 }
 
+struct BTerms {
+    const BTerm* __restrict__ t;
+    __device__ __forceinline__ uint64_t x(int i) const { return t[i].x; }
+    __device__ __forceinline__ uint64_t z(int i) const { return t[i].z; }
+    __device__ __forceinline__ double re(int i) const { return t[i].cre; }
+    __device__ __forceinline__ double im(int i) const { return t[i].cim; }
+};
+
 // lam[j] = sum_t c_t (-1)^popc(z_t & (j ^ x_t)) psi[j ^ x_t] for j in [j0, j1),
 // and the FP64 partial of <psi|lam> over the range (lam as stored).  psi was
-// written by other CTAs of this launch: it is read through L2 (ld.cg).
+// written by other CTAs of this launch: it is read through L2 (ld.cg).  Ranges
+// of whole 2048-amplitude chunks take eight amplitudes per thread (pauli.cuh).
+template <typename V, bool CPLX>
+__device__ __noinline__ void ham_chunks(const V* psi, V* lam, const BTerms tm, int nterms, uint64_t j0, uint64_t j1,
+                                        double& er, double& ei) {
+    const uint64_t lanes = (j1 - j0) / kPauliU;
+    for (uint64_t q = threadIdx.x; q < lanes; q += blockDim.x) {
+        const uint64_t lo = q & ((uint64_t(1) << kPauliShift) - 1);
+        const uint64_t base = j0 + (q >> kPauliShift) * kPauliChunk + lo;
+        double re[kPauliU], im[kPauliU];
+        pauli8<CPLX>(tm, nterms, base, [&](uint64_t i) { return __ldcg(psi + i); }, re, im);
+#pragma unroll
+        for (int u = 0; u < kPauliU; ++u) {
+            const uint64_t j = base | (uint64_t(u) << kPauliShift);
+            const V lv = mk<V>(re[u], im[u]);
+            lam[j] = lv;
+            const V a = __ldcg(psi + j);
+            er += double(a.x) * double(lv.x) + double(a.y) * double(lv.y);
+            ei += double(a.x) * double(lv.y) - double(a.y) * double(lv.x);
+        }
+    }
+}
+
 template <typename V>
 __device__ void ham_range(V* __restrict__ pl, const BInst& I, const BTerm* __restrict__ tm, uint64_t j0, uint64_t j1,
                           double* __restrict__ out) {
@@ -94,28 +125,29 @@ __device__ void ham_range(V* __restrict__ pl, const BInst& I, const BTerm* __res
     const V* psi = pl;
     V* lam = pl + N;
     double er = 0.0, ei = 0.0;
-    for (uint64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-        double re = 0.0, im = 0.0;
-        int t = 0;
-        while (t < I.nterms) {
-            const uint64_t x = tm[t].x;
-            const uint64_t src = j ^ x;
-            const V a = __ldcg(psi + src);
-            double sr = 0.0, si = 0.0;
-            for (; t < I.nterms && tm[t].x == x; ++t) {
+    if (((j0 | j1) & (kPauliChunk - 1)) == 0) {
+        bool cplx = false;
+        for (int t = 0; t < I.nterms; ++t) cplx = cplx || tm[t].cim != 0.0;
+        if (cplx) ham_chunks<V, true>(psi, lam, BTerms{tm}, I.nterms, j0, j1, er, ei);
+        else ham_chunks<V, false>(psi, lam, BTerms{tm}, I.nterms, j0, j1, er, ei);
+    } else {
+        for (uint64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
+            double re = 0.0, im = 0.0;
+            for (int t = 0; t < I.nterms; ++t) {
+                const uint64_t src = j ^ tm[t].x;
+                const V a = __ldcg(psi + src);
                 const bool neg = __popcll(tm[t].z & src) & 1;
-                sr += neg ? -tm[t].cre : tm[t].cre;
-                si += neg ? -tm[t].cim : tm[t].cim;
+                const double sr = neg ? -tm[t].cre : tm[t].cre, si = neg ? -tm[t].cim : tm[t].cim;
+                const double ar = double(a.x), ai = double(a.y);
+                re += sr * ar - si * ai;
+                im += sr * ai + si * ar;
             }
-            const double ar = double(a.x), ai = double(a.y);
-            re += sr * ar - si * ai;
-            im += sr * ai + si * ar;
+            const V lv = mk<V>(re, im);
+            lam[j] = lv;
+            const V u = __ldcg(psi + j);
+            er += double(u.x) * double(lv.x) + double(u.y) * double(lv.y);
+            ei += double(u.x) * double(lv.y) - double(u.y) * double(lv.x);
         }
-        const V lv = mk<V>(re, im);
-        lam[j] = lv;
-        const V u = __ldcg(psi + j);
-        er += double(u.x) * double(lv.x) + double(u.y) * double(lv.y);
-        ei += double(u.x) * double(lv.y) - double(u.y) * double(lv.x);
     }
     const double2 s = block_sum(er, ei);
     if (threadIdx.x == 0) {
