@@ -42,6 +42,27 @@ def _min_k(precision: str) -> int:
     return 9 if precision == "double" else 10
 
 
+def item_sizes(ns: Sequence[int], caps: Tuple[int, int], sms: int) -> Tuple[int, int]:
+    """(tiles per item, amplitudes per lam = H psi item) of a batch of problems
+    of `ns` qubits: the largest powers of two, up to the defaults, that still
+    give every SM about two register items and four lam = H psi items a round.
+    A batch that fills the GPU anyway keeps the defaults (fewer waits and
+    table stagings per tile).  32 MaxCut instances of 10..20 qubits, complex64,
+    caps (13, 13) (B200): 16 / 8 / 4 / 2 / 1 tiles an item 6.18 / 3.7 / 3.1 / 3.4 /
+    4.0 ms; 128 of them 12.0 / 11.8 ms at 16 / 8; complex128, caps (11, 11):
+    6.9 / 5.6 / 5.6 ms at 16 / 8 / 4."""
+    tiles = sum(max(1, (1 << n) >> min(caps[0], n)) for n in ns)
+    amps = sum(1 << n for n in ns)
+
+    def fit(per: float, least: int, most: int) -> int:
+        k = least
+        while 2 * k <= most and 1.5 * k <= per:
+            k *= 2
+        return k
+
+    return fit(tiles / (2 * sms), 1, 16), fit(amps / (4 * sms), 1 << 11, 1 << 14)
+
+
 class PersistentBatch:
     """problems: [(engine, params)] with params one row of the engine's
     circuit parameters.  Every engine must have the batch's precision and

@@ -83,7 +83,7 @@ class UnevenQAOABatch:
         self.captured_launches = 0
         self.graph = None
         if mode == "persistent":
-            from .persistent import PersistentBatch, batch_key
+            from .persistent import batch_key
             tuner = tuner or Autotuner()
             dev = torch.device("cuda", device_id)
             self.caps = caps
@@ -91,9 +91,7 @@ class UnevenQAOABatch:
                 self.caps = tuner.lookup_adjoint(batch_key(torch.cuda.get_device_name(dev), precision, label))
             self.engines = [BatchedAdjoint(qaoa_circuit(n, edges, p), maxcut_observable(n, edges), precision,
                                            device_id) for n, edges, p, _ in instances]
-            self.persistent = PersistentBatch([(e, np.asarray(prm)) for e, (_, _, _, prm) in
-                                               zip(self.engines, instances)], precision, device_id, caps=self.caps,
-                                              jit_min_qubits=jit_min_qubits)
+            self.persistent = self._make_persistent(precision, device_id, self.caps)
             self.caps = self.persistent.caps
             self.dev = self.persistent.dev
             return
@@ -122,21 +120,26 @@ class UnevenQAOABatch:
         self.nstreams = streams
         self.graph = None
 
+    def _make_persistent(self, precision: str, device_id: int, caps: Optional[Tuple[int, int]]):
+        from .persistent import DEFAULT_CAPS, PersistentBatch, item_sizes
+        sms = torch.cuda.get_device_properties(device_id).multi_processor_count
+        tiles, amps = item_sizes([e.n for e in self.engines], caps or DEFAULT_CAPS[precision], sms)
+        return PersistentBatch([(e, np.asarray(prm)) for e, (_, _, _, prm) in zip(self.engines, self.instances)],
+                               precision, device_id, caps=caps, tiles_per_item=tiles, amps_per_ham_item=amps,
+                               jit_min_qubits=self.jit_min_qubits)
+
     def tune_caps(self, label: str, tuner: Optional[Autotuner] = None):
         """Persistent mode: time every tile-width cap candidate on this batch,
         store the fastest under the "batch" key of `label` and rebuild the
         batch with it; returns (caps, ms, trials)."""
-        from .persistent import PersistentBatch, batch_key, tune
+        from .persistent import batch_key, tune
         if self.mode != "persistent":
             raise ValueError("tune_caps applies to mode='persistent'")
         prec = self.persistent.precision
-        probs = [(e, np.asarray(prm)) for e, (_, _, _, prm) in zip(self.engines, self.instances)]
         key = batch_key(torch.cuda.get_device_name(self.dev), prec, label)
         self.persistent = None
-        jm = self.jit_min_qubits
-        best, ms, trials = tune(lambda caps: PersistentBatch(probs, prec, self.dev.index, caps=caps,
-                                                             jit_min_qubits=jm), prec, key, tuner)
-        self.persistent = PersistentBatch(probs, prec, self.dev.index, caps=best, jit_min_qubits=jm)
+        best, ms, trials = tune(lambda caps: self._make_persistent(prec, self.dev.index, caps), prec, key, tuner)
+        self.persistent = self._make_persistent(prec, self.dev.index, best)
         self.caps = best
         self.graph = None
         return best, ms, trials
