@@ -569,25 +569,33 @@ int launch_jit(V* vec, PlanLaunch& L, int R, const V* hm, const V* mats, double*
     return 1;
 }
 
-// Register bits per thread of generated passes: the generic kernel's (4 for
-// complex128, 5 for complex64) unless QS_JIT_REG_BITS says otherwise (4 or 5).
-inline int jit_reg_bits(int generic_r) {
+// Register bits per thread of generated passes.  complex128: 4, as the generic
+// kernel.  complex64: 4 where a tile of 2^k amplitudes then has at most 256
+// threads (k <= 12), else the generic kernel's 5.  Half the amplitudes per
+// thread leave registers for three times the warps, and passes of complex64 are
+// bound by the issue of dependent instructions, not by their relayouts.  4
+// against 5 (B200, k = 12): 30-qubit spread circuit of 1000 gates 147.6 against
+// 163.2 ms (139.2 at nlow = 5), 28 qubits, 400 gates 14.4 against 15.6 ms, 24
+// qubits 643 against 845 us, 18 qubits 27 against 37 us.  QS_JIT_REG_BITS (4 or
+// 5) overrides both.
+inline int jit_reg_bits(int generic_r, int k) {
     static const int env_r = [] {
         const char* e = getenv("QS_JIT_REG_BITS");
         const int v = e && *e ? atoi(e) : 0;
         return (v == 4 || v == 5) ? v : 0;
     }();
-    return env_r ? env_r : generic_r;
+    if (env_r) return env_r;
+    return generic_r == 5 && k <= 12 ? 4 : generic_r;
 }
 
 template <typename V, int R, bool EXP, bool BIG>
 int launch_reg_k(V* vec, int n, const qs_pass& ps, const qs_op* ops, const V* mats, double* partials, cudaStream_t st,
                  const V* hm = nullptr) {
     const int nb = sizeof(V) == 16 ? 3 : 4;  // bank-group bits of a shared-memory phase
-    const int RJ = jit_reg_bits(R);
+    const int RJ = jit_reg_bits(R, ps.k);
     qs_pass rest = ps;
     std::vector<qs_op> rest_ops;
-    if (!EXP && RJ != R && ps.k - RJ >= 5 && ps.k - RJ <= 8) {
+    if (RJ != R && ps.k - RJ >= 5 && ps.k - RJ <= 8 && hm != nullptr && jit::mode() != QS_JIT_OFF) {
         // a generated pass with its own register width has its own plan; from
         // the first launch that is not ready on, the generic kernel's plan of
         // the remaining ops takes over
@@ -609,7 +617,7 @@ int launch_reg_k(V* vec, int n, const qs_pass& ps, const qs_op* ops, const V* ma
     if (!plan) return QS_EINVAL;
     for (const auto& L : plan->launches) {
         const RegArgs& args = L->args;
-        if (EXP || RJ == R) {
+        if (RJ == R) {
             const int jr = launch_jit<V>(vec, *L, R, hm, mats, partials, st);
             if (jr < 0) return jr;
             if (jr == 1) continue;
@@ -802,7 +810,7 @@ extern "C" int qs_jit_pass_source(int n, int dtype, const qs_pass* pass, const q
     // pair passes (adjoint) carry EXPECT ops; their partials buffer is not touched here
     int rc = validate_pass(*pass, n, ops, nops_total, mats_count, pass->pair > 0, INT64_MAX / 4);
     if (rc) return rc;
-    const int R = jit_reg_bits(dtype == QS_C128 ? reg_bits<double2>() : reg_bits<float2>());
+    const int R = jit_reg_bits(dtype == QS_C128 ? reg_bits<double2>() : reg_bits<float2>(), pass->k);
     const int nT = pass->k - R;
     if (!(nT >= 5 && nT <= 8 && pass->nlow >= 5)) {
         set_error("qs_jit_pass_source: tile 2^%d / nlow %d is not a register tile", pass->k, pass->nlow);

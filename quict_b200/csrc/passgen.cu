@@ -566,12 +566,15 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
         const char* e = getenv("QS_JIT_THREADS_PER_SM");
         return e && *e ? atoi(e) : 0;
     }();
-    // 512 threads per SM; plain complex64 state-vector passes (no per-instance
-    // tables, no EXPECT ops) 256, i.e. the whole register file for 64-thread
-    // CTAs: on the 30-qubit spread circuit (B200, k = 11) 211.6 -> 189.7 ms
-    // (384: 208.2 ms).  complex128 passes are fastest at 512 (298 ms at 640,
-    // 344 ms at 768).
-    const int target = env_target > 0 ? env_target : (!C128 && !batched && a.nexp == 0 ? 256 : 512);
+    // 512 threads per SM; plain complex64 passes (no per-instance tables, no
+    // EXPECT ops) with 4 register bits 768 (30-qubit spread circuit, k = 12,
+    // nlow 6, B200: 151.2 -> 148.1 ms; 28 qubits 14.5, 14.4 and at 1024 14.7
+    // ms), with 5 register bits 256, i.e. the whole register file for 64-thread
+    // CTAs (k = 11: 211.6 -> 189.7 ms; 384: 208.2 ms).  complex128 passes are
+    // fastest at 512 (k = 12: 261 ms; 295 ms at 256; k = 10 at 640: 275 against
+    // 269 ms).
+    const bool plain64 = !C128 && !batched && a.nexp == 0;
+    const int target = env_target > 0 ? env_target : !plain64 ? 512 : R == 4 ? 768 : 256;
     const int minb = threads >= target ? 1 : target / threads;
     SrcBuf g;
     g.add("// generated fused pass: n=%d K=%d L=%d R=%d stages=%d ops=%d expect=%d batched=%d\n", a.n, K, L, R,

@@ -63,13 +63,16 @@ def default_knobs(esize: int, n: Optional[int] = None) -> Knobs:
       complex128, k = 10 / 11 / 12: 14 qubits 27 / 27 / 37 us, 18 qubits 37 / 35 /
         43 us, 22 qubits 222 / 227 / 265 us, 24 qubits 1243 / 976 / 1104 us, 26
         qubits 4.07 / 3.68 / 3.82 ms, 28 qubits 19.4 / 16.0 / 15.9 ms
-      complex64, k = 11 / 12 / 13: 14 qubits 31 / 33 / 39 us, 18 qubits 41 / 37 / 41
-        us, 22 qubits 160 / 150 / 162 us, 24 qubits 536 / 552 / 459 us, 26 qubits
-        2.09 / 1.99 / 1.92 ms, 28 qubits 8.36 / 8.33 / 8.08 ms
+      complex64, k = 11 / 12 / 13: 14 qubits 23 / 24 / 39 us, 18 qubits 29 / 27 / 41
+        us, 20 qubits 45 / 43 us at 11 / 12, 22 qubits 129 / 138 / 162 us, 24
+        qubits 497 / 552 / 459 us, 25 qubits (300 gates) 1316 / 1238 us at 12 / 13,
+        26 qubits 1.92 / 1.91 / 1.92 ms, 28 qubits 8.47 / 8.02 / 8.08 ms; on 400
+        gates of the spread circuit 15.5 / 14.4 / 23.3 ms
 
     On a small state narrow tiles give more SMs a tile; a state that fits the
-    L2 cache is read cheaply, so several CTAs per SM are worth more passes;
-    beyond it every pass saved counts.  Without `n` (and for density matrices,
+    L2 cache is read cheaply, so several CTAs per SM are worth more passes; just
+    beyond it a pass saved counts most; on the largest the widest complex64
+    tiles, one CTA per SM, lose more on dense passes than they save.  Without `n` (and for density matrices,
     whose 12-qubit noisy runs took 2.97 ms at k = 12 and 3.20 ms at k = 11): the
     widest tiles."""
     if n is None:
@@ -77,7 +80,7 @@ def default_knobs(esize: int, n: Optional[int] = None) -> Knobs:
     elif esize == 16:
         k = 11 if n < 27 else 12
     else:
-        k = 11 if n < 17 else 12 if n < 24 else 13
+        k = 11 if n < 17 else 13 if 24 <= n < 26 else 12
     return Knobs(k, 5, 2)
 
 
