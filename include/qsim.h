@@ -219,6 +219,11 @@ int qs_jit_compile_check(const char* src, int64_t* cubin_bytes);
 int qs_jit_pass_source(int n, int dtype, const qs_pass* pass, const qs_op* ops, int64_t nops_total,
                        const void* mats_host, int64_t mats_count, int launch_index, char* out,
                        size_t out_size, int64_t* src_len);
+/* The same launch's parameter block (`struct P` of its source): *bytes <- its
+ * size; up to out_size bytes are copied to `out` (may be NULL). */
+int qs_jit_pass_params(int n, int dtype, const qs_pass* pass, const qs_op* ops, int64_t nops_total,
+                       const void* mats_host, int64_t mats_count, int launch_index, void* out,
+                       size_t out_size, int64_t* bytes);
 
 /* ---- differentiation / observables ---------------------------------------- */
 /* Backward-sweep pass of the adjoint method: every QS_OP_MAT / DIAG / ANTI /

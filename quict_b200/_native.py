@@ -160,6 +160,8 @@ SIGNATURES = {
     "qs_jit_compile_check": (_i, [C.c_char_p, C.POINTER(C.c_int64)]),
     "qs_jit_pass_source": (_i, [_i, _i, C.POINTER(qs_pass), C.POINTER(qs_op), _i64, _vp, _i64, _i, C.c_char_p, _sz,
                                 C.POINTER(C.c_int64)]),
+    "qs_jit_pass_params": (_i, [_i, _i, C.POINTER(qs_pass), C.POINTER(qs_op), _i64, _vp, _i64, _i, _vp, _sz,
+                                C.POINTER(C.c_int64)]),
 }
 
 _lib = None

@@ -800,12 +800,15 @@ extern "C" int qs_adjoint_pair_ex(void* psilam, int n, int dtype, const qs_pass*
     return QS_OK;
 }
 
-extern "C" int qs_jit_pass_source(int n, int dtype, const qs_pass* pass, const qs_op* ops, int64_t nops_total,
-                                  const void* mats_host, int64_t mats_count, int launch_index, char* out,
-                                  size_t out_size, int64_t* src_len) {
+namespace {
+
+// Launch `launch_index` of one register pass as its generated kernel (source,
+// parameter block), without a device.
+int generated_launch(const char* who, int n, int dtype, const qs_pass* pass, const qs_op* ops, int64_t nops_total,
+                     const void* mats_host, int64_t mats_count, int launch_index, JitPass& jp) {
     QS_REQUIRE(n >= 1 && n <= 40, "qubit count %d outside [1, 40]", n);
     QS_REQUIRE(valid_dtype(dtype), "bad dtype %d", dtype);
-    QS_REQUIRE(pass != nullptr && mats_host != nullptr && src_len != nullptr, "null argument");
+    QS_REQUIRE(pass != nullptr && mats_host != nullptr, "null argument");
     QS_REQUIRE(launch_index >= 0, "negative launch index");
     // pair passes (adjoint) carry EXPECT ops; their partials buffer is not touched here
     int rc = validate_pass(*pass, n, ops, nops_total, mats_count, pass->pair > 0, INT64_MAX / 4);
@@ -813,35 +816,57 @@ extern "C" int qs_jit_pass_source(int n, int dtype, const qs_pass* pass, const q
     const int R = jit_reg_bits(dtype == QS_C128 ? reg_bits<double2>() : reg_bits<float2>(), pass->k);
     const int nT = pass->k - R;
     if (!(nT >= 5 && nT <= 8 && pass->nlow >= 5)) {
-        set_error("qs_jit_pass_source: tile 2^%d / nlow %d is not a register tile", pass->k, pass->nlow);
+        set_error("%s: tile 2^%d / nlow %d is not a register tile", who, pass->k, pass->nlow);
         return QS_ENOTSUP;
     }
     static thread_local RegArgs args;
     std::vector<int> rem(pass->op_count);
     for (int i = 0; i < pass->op_count; ++i) rem[i] = i;
-    JitPass jp;
-    bool ok = false;
     for (int li = 0; li <= launch_index; ++li) {
         if (rem.empty()) {
-            set_error("qs_jit_pass_source: the pass has %d launches", li);
+            set_error("%s: the pass has %d launches", who, li);
             return QS_EINVAL;
         }
         if (build_reg(*pass, ops, rem, n, R, dtype == QS_C128 ? 3 : 4, args) <= 0) {
-            set_error("qs_jit_pass_source: an op does not fit a register tile");
+            set_error("%s: an op does not fit a register tile", who);
             return QS_EINVAL;
         }
-        if (li == launch_index)
-            ok = gen_pass(&args, R, dtype == QS_C128, mats_host, jp, true);
     }
-    if (!ok) {
-        set_error("qs_jit_pass_source: this launch is not generated (batched, EXPECT ops or parameters too large)");
+    if (!gen_pass(&args, R, dtype == QS_C128, mats_host, jp, true)) {
+        set_error("%s: this launch is not generated (batched, EXPECT ops or parameters too large)", who);
         return QS_ENOTSUP;
     }
+    return QS_OK;
+}
+
+}  // namespace
+
+extern "C" int qs_jit_pass_source(int n, int dtype, const qs_pass* pass, const qs_op* ops, int64_t nops_total,
+                                  const void* mats_host, int64_t mats_count, int launch_index, char* out,
+                                  size_t out_size, int64_t* src_len) {
+    QS_REQUIRE(src_len != nullptr, "null argument");
+    JitPass jp;
+    const int rc = generated_launch("qs_jit_pass_source", n, dtype, pass, ops, nops_total, mats_host, mats_count,
+                                    launch_index, jp);
+    if (rc) return rc;
     *src_len = int64_t(jp.src.size());
     if (out != nullptr && out_size > 0) {
         const size_t k = jp.src.size() < out_size - 1 ? jp.src.size() : out_size - 1;
         memcpy(out, jp.src.data(), k);
         out[k] = 0;
     }
+    return QS_OK;
+}
+
+extern "C" int qs_jit_pass_params(int n, int dtype, const qs_pass* pass, const qs_op* ops, int64_t nops_total,
+                                  const void* mats_host, int64_t mats_count, int launch_index, void* out,
+                                  size_t out_size, int64_t* bytes) {
+    QS_REQUIRE(bytes != nullptr, "null argument");
+    JitPass jp;
+    const int rc = generated_launch("qs_jit_pass_params", n, dtype, pass, ops, nops_total, mats_host, mats_count,
+                                    launch_index, jp);
+    if (rc) return rc;
+    *bytes = int64_t(8 * jp.params.size());
+    if (out != nullptr) memcpy(out, jp.params.data(), out_size < 8 * jp.params.size() ? out_size : 8 * jp.params.size());
     return QS_OK;
 }

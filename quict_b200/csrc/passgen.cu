@@ -237,7 +237,7 @@ struct Normaliser {
     void run() {
         Cx total(1, 0);
         double up = 0, down = 0, held = 0;                 // scalars so far; factors on their way to a taker
-        std::vector<double> raised(size_t(a.nops), 0.0);  // by the scalar taken out of each op
+        std::vector<double> raised(size_t(a.nops), 0.0);  // by the scalars that appear at each op
         std::vector<double> release(size_t(a.nops), 0.0);
         for (int o = 0; o < a.nops; ++o) {
             held -= release[size_t(o)];
@@ -254,7 +254,9 @@ struct Normaliser {
             int best_cost = mat_cost(best.data(), D);
             const double ls = std::log2(std::abs(s));
             const double u_up = std::max(0.0, -ls), u_down = std::max(0.0, ls);
-            double u_held = 0;
+            // a factor inverted by an exchange leaves the scalar 1 / d once it is
+            // taken (X diag(1, d) = d diag(1, 1/d) X), for the rest of the launch
+            double u_held = 0, i_up = 0, i_down = 0;
             if (best_cost >= mat_cost(u.data(), D)) continue;
             std::vector<int> to(size_t(M), -1), tob(size_t(M), 0);
             std::vector<char> inv(size_t(M), 0);
@@ -286,13 +288,19 @@ struct Normaliser {
                 to[size_t(i)] = p;
                 tob[size_t(i)] = bit;
                 inv[size_t(i)] = iv;
-                u_held += std::abs(std::log2(std::abs(d2[size_t(i)])));
+                const double ld = std::log2(std::abs(d2[size_t(i)]));
+                u_held += std::abs(ld);
+                if (iv) {
+                    i_up += std::max(0.0, -ld);
+                    i_down += std::max(0.0, ld);
+                }
             }
-            if (up + u_up > max_up || down + u_down + held + u_held > max_down) continue;
-            up += u_up;
-            down += u_down;
+            // (written so that a value that is not finite refuses the op)
+            if (!(up + u_up + i_up + held + u_held <= max_up && down + u_down + i_down + held + u_held <= max_down)) continue;
+            up += u_up + i_up;
+            down += u_down + i_down;
             held += u_held;
-            raised[size_t(o)] = -ls;
+            raised[size_t(o)] += u_up;
             u = best;
             total = exact_mul(total, s);
             for (int i = 0; i < M; ++i) {
@@ -300,6 +308,7 @@ struct Normaliser {
                 Cx f = d[size_t(i)];
                 if (inv[size_t(i)]) {  // X diag(1, d) = d diag(1, 1/d) X
                     total = exact_mul(total, f);
+                    raised[size_t(to[size_t(i)])] += std::max(0.0, -std::log2(std::abs(f)));
                     f = exact_div(Cx(1, 0), f);
                 }
                 const int p = to[size_t(i)];
@@ -315,7 +324,7 @@ struct Normaliser {
         for (int o = a.nops - 1; o >= 0; --o) {
             const KOp& op = a.ops[o];
             const double low = after;
-            after += std::max(0.0, raised[size_t(o)]);
+            after += raised[size_t(o)];
             if (low > max_down) break;
             if (controlled(op) || (op.code != QS_OP_MAT && op.code != QS_OP_DIAG)) continue;
             std::vector<Cx> v = m[size_t(o)];
