@@ -80,17 +80,22 @@ std::string thread_xor_expr(const uint32_t* img, int nT) {
 //   - D_i moves forward along its bit (through diagonals and controls, across
 //     plain exchanges) into the next uncontrolled op on that bit; d_i = 1 when
 //     no op takes it.
-// Row and scalar factors leave every product's relative rounding error as it
-// is; only the range grows, so the launch's factors are bounded (see run).
-// Which entry becomes 1 depends on the pattern of zeros and on classes that
-// hold for every value (real, imaginary, equal up to sign), not on the values'
-// sizes: new parameters of a circuit reuse its compiled kernels.
+// The factors are products and quotients in extended precision (64 significand
+// bits), rounded once into the parameter block; a coefficient is never changed
+// by more than that rounding.  Row and scalar factors leave every product's
+// relative rounding error as it is; only the range grows, so the launch's
+// factors are bounded (see run).
+// Which entry becomes 1, and the class of every other one, follows from the
+// classes of the matrices' own entries and from exact equalities between them,
+// never from the size or the last bits of a result: new parameters of a circuit
+// reuse its compiled kernels.
 // 30-qubit spread circuit of 1000 gates (B200): 3316 -> 2706 multiply-add
 // instructions per amplitude, complex128 318.3 -> 276.3 ms, complex64 202.4 ->
 // 179.0 ms; 25 qubits, 300 gates, complex64 2.04 -> 1.84 ms, its error against
 // 64-bit arithmetic 3.8e-7 -> 3.5e-7 (fewer roundings).  Per-instance tables
 // and adjoint passes keep their matrices.
-using Cx = std::complex<double>;
+#pragma nv_diag_suppress 20208  // long double: host code only here
+using Cx = std::complex<long double>;
 
 // 0, 1, -1, general (3), real (4), imaginary (5)
 template <typename T>
@@ -99,58 +104,101 @@ int value_class(T x, T y) {
     return x == 0 ? 5 : 3;
 }
 
+// A matrix entry, its class (what the generated code may assume about it) and
+// the size of the rounding it came with: half a unit in the last place of its
+// matrix's largest entry.
+struct Entry {
+    Cx z;
+    int cl;
+    long double err;
+};
+inline bool is_real(int cl) { return cl == 1 || cl == 2 || cl == 4; }
+const Entry kOne{Cx(1, 0), 1, 0};
+
+int mul_class(int a, int b) {
+    if (a == 0 || b == 0) return 0;
+    if (a == 1 || b == 1) return a == 1 ? b : a;
+    if (a == 2 && b == 2) return 1;
+    if (a == 3 || b == 3) return 3;
+    return is_real(a) == is_real(b) ? 4 : 5;
+}
+// an entry times a factor
+Entry mul(const Entry& a, const Entry& f) {
+    const int cl = mul_class(a.cl, f.cl);
+    const long double x = a.z.real(), y = a.z.imag(), u = f.z.real(), v = f.z.imag();
+    const long double err = a.err == 0 ? 0 : a.err * std::max(std::abs(u), std::abs(v));
+    if (cl == 0) return {Cx(0, 0), 0, err};
+    if (is_real(f.cl)) return {Cx(x * u, y * u), cl, err};
+    if (is_real(a.cl)) return {Cx(x * u, x * v), cl, err};
+    return {Cx(x * u - y * v, x * v + y * u), cl, err};
+}
+// Two entries that are the same number: merged matrices hold such pairs as sums
+// rounded in different orders.  Each component is compared by itself (that of an
+// angle of 2 pi, next to 0, counts), and a pair taken for equal changes its
+// matrix by no more than the roundings it came with.
+bool same(const Entry& a, const Entry& b, const Cx& bz) {
+    const auto near = [e = a.err + b.err](long double x, long double u) {
+        const long double d = std::abs(x - u);
+        return d == 0 || (d <= e && d <= 0x1p-44L * std::abs(u) && x != 0);
+    };
+    return near(a.z.real(), bz.real()) && near(a.z.imag(), bz.imag());
+}
+// class of a / b: +-1 and +-i where the entries are the same up to that factor
+int div_class(const Entry& a, const Entry& b) {
+    if (a.cl == 0) return 0;
+    if (same(a, b, b.z)) return 1;
+    if (same(a, b, -b.z)) return 2;
+    if (b.cl == 1 || b.cl == 2) return a.cl;
+    if (a.cl == 3 || b.cl == 3) {
+        const Cx t(-b.z.imag(), b.z.real());
+        return same(a, b, t) || same(a, b, -t) ? 5 : 3;
+    }
+    return is_real(a.cl) == is_real(b.cl) ? 4 : 5;
+}
+Entry div(const Entry& a, const Entry& b) {
+    const int cl = div_class(a, b);
+    const long double x = a.z.real(), y = a.z.imag(), u = b.z.real(), v = b.z.imag();
+    Cx q(0, 0);
+    if (cl == 1 || cl == 2) q = Cx(cl == 1 ? 1 : -1, 0);
+    else if (cl == 4) q = Cx(is_real(b.cl) ? x / u : y / v, 0);
+    else if (cl == 5 && a.cl == 3) q = Cx(0, same(a, b, Cx(-v, u)) ? 1 : -1);
+    else if (cl == 5) q = Cx(0, is_real(b.cl) ? y / u : -x / v);
+    else if (cl == 3 && is_real(b.cl)) q = Cx(x / u, y / u);
+    else if (cl == 3) q = Cx((x * u + y * v) / (u * u + v * v), (y * u - x * v) / (u * u + v * v));
+    return {q, cl, 0};  // (quotients are factors or final entries)
+}
+double log2_abs(const Entry& e) { return double(std::log2(std::abs(e.z))); }
+
 // Instructions per amplitude of one row: the first term may be a unit entry
 // (taken as is), which the generated code puts first.
-int row_cost(const Cx* m, int D) {
+struct RowCost {
     int c = 0;
-    bool unit = false, any = false;
-    for (int i = 0; i < D; ++i) {
-        const int cl = value_class(m[i].real(), m[i].imag());
-        if (cl == 0) continue;
-        any = true;
+    bool unit = false;
+    void add(int cl) {
+        if (cl == 0) return;
         if (cl <= 2) unit = true;
         c += cl == 3 ? 4 : 2;
     }
-    return any && unit ? c - 2 : c;
-}
-int mat_cost(const Cx* m, int D) {  // summed over the rows
+    int total() const { return unit ? c - 2 : c; }
+};
+int mat_cost(const Entry* m, int D) {  // summed over the rows
     int c = 0;
-    for (int r = 0; r < D; ++r) c += row_cost(m + r * D, D);
+    for (int r = 0; r < D; ++r) {
+        RowCost row;
+        for (int i = 0; i < D; ++i) row.add(m[r * D + i].cl);
+        c += row.total();
+    }
     return c;
-}
-
-// Products and quotients that keep the classes: exact zeros stay, and a part
-// that vanishes, or a quotient that is +-1, up to the rounding of this very
-// operation is what it is for every value (a phase that cancels), so it is set;
-// a class that came and went with the last bit would mean another kernel.
-constexpr double kClassTol = 0x1p-48;
-Cx settle(Cx q) {
-    const double r = std::abs(q.real()), i = std::abs(q.imag());
-    if (i <= kClassTol * r) return Cx(q.real(), 0.0);
-    if (r <= kClassTol * i) return Cx(0.0, q.imag());
-    return q;
-}
-Cx exact_mul(Cx a, Cx b) {
-    if (a.imag() == 0 && b.imag() == 0) return Cx(a.real() * b.real(), 0.0);
-    return settle(Cx(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()));
-}
-Cx exact_div(Cx a, Cx b) {
-    if (a == b) return Cx(1, 0);
-    if (a == -b) return Cx(-1, 0);
-    if (a == Cx(0, 0)) return Cx(0, 0);
-    const Cx q = b.imag() == 0 ? Cx(a.real() / b.real(), a.imag() / b.real()) : settle(a / b);
-    if (q.imag() == 0 && std::abs(std::abs(q.real()) - 1.0) <= kClassTol) return Cx(q.real() > 0 ? 1 : -1, 0);
-    return q;
 }
 
 struct Normaliser {
     const RegArgs& a;
-    std::vector<std::vector<Cx>>& m;  // per op, slot order (MAT: row-major D x D; DIAG: 2^m entries)
+    std::vector<std::vector<Entry>>& m;  // per op, slot order (MAT: row-major D x D; DIAG: 2^m entries)
     // log2 bounds on how far taking factors out may raise (up) and lower (down)
     // the amplitudes between the launch's load and its store
     const double max_up, max_down;
 
-    Normaliser(const RegArgs& a_, std::vector<std::vector<Cx>>& m_, double max_up_, double max_down_)
+    Normaliser(const RegArgs& a_, std::vector<std::vector<Entry>>& m_, double max_up_, double max_down_)
         : a(a_), m(m_), max_up(max_up_), max_down(max_down_) {}
 
     const KStage& stage_of(int o) const {
@@ -179,8 +227,8 @@ struct Normaliser {
         const KOp& op = a.ops[o];
         if (op.code != QS_OP_DIAG || controlled(op)) return false;
         if (op.nh > 0) return true;
-        for (const Cx& z : m[size_t(o)])
-            if (value_class(z.real(), z.imag()) != 3) return false;
+        for (const Entry& z : m[size_t(o)])
+            if (z.cl != 3) return false;
         return true;
     }
     // The op that takes a factor diag(1, d) of tile bit b from op o, the bit it
@@ -212,10 +260,10 @@ struct Normaliser {
         return -1;
     }
     // m[p] <- m[p] diag(1, d) on index bit ib (columns; entries of a diagonal)
-    void take(std::vector<Cx>& v, bool diag, int ib, Cx d) const {
+    void take(std::vector<Entry>& v, bool diag, int ib, const Entry& d) const {
         const size_t D = diag ? v.size() : size_t(1) << (ctz(v.size()) / 2);
         for (size_t e = 0; e < v.size(); ++e)
-            if (((e & (D - 1)) >> ib) & 1) v[e] = exact_mul(v[e], d);
+            if (((e & (D - 1)) >> ib) & 1) v[e] = mul(v[e], d);
     }
     static int ctz(size_t x) {
         int c = 0;
@@ -223,19 +271,25 @@ struct Normaliser {
         return c;
     }
     // best cost of a matrix whose rows may all be scaled (an estimate)
-    static int scaled_cost(std::vector<Cx> v) {
+    static int scaled_cost(const std::vector<Entry>& v) {
         const int D = 1 << (ctz(v.size()) / 2);
+        if (D > 4) return mat_cost(v.data(), D);
+        int cost = 0;
         for (int r = 0; r < D; ++r) {
-            const Cx z = v[size_t(r * D + r)];
-            if (D > 4 || z == Cx(0, 0)) continue;
-            for (int c = 0; c < D; ++c) v[size_t(r * D + c)] = exact_div(v[size_t(r * D + c)], z);
+            const Entry& z = v[size_t(r * D + r)];
+            RowCost row;
+            for (int c = 0; c < D; ++c) {
+                const Entry& e = v[size_t(r * D + c)];
+                row.add(z.cl == 0 ? e.cl : div_class(e, z));
+            }
+            cost += row.total();
         }
-        return mat_cost(v.data(), D);
+        return cost;
     }
 
     // Take factors out of every uncontrolled dense op on one or two bits.
     void run() {
-        Cx total(1, 0);
+        Entry total = kOne;
         double up = 0, down = 0, held = 0;                 // scalars so far; factors on their way to a taker
         std::vector<double> raised(size_t(a.nops), 0.0);  // by the scalars that appear at each op
         std::vector<double> release(size_t(a.nops), 0.0);
@@ -243,52 +297,49 @@ struct Normaliser {
             held -= release[size_t(o)];
             const KOp& op = a.ops[o];
             if (op.code != QS_OP_MAT || controlled(op)) continue;
-            std::vector<Cx>& u = m[size_t(o)];
+            std::vector<Entry>& u = m[size_t(o)];
             const int M = popc_c(op.mask), D = 1 << M;
             if (M > 2) continue;
             const KStage& S = stage_of(o);
-            const Cx s = u[0];
+            const Entry s = u[0];
             if (!usable(s, u)) continue;
-            std::vector<Cx> d(size_t(M), Cx(1, 0));
-            std::vector<Cx> best = scaled(u, s, d);
-            int best_cost = mat_cost(best.data(), D);
-            const double ls = std::log2(std::abs(s));
+            int own = 0;  // index bits whose d_i is taken out
+            int best_cost = rows_cost(u, M, own);
+            const double ls = log2_abs(s);
             const double u_up = std::max(0.0, -ls), u_down = std::max(0.0, ls);
             // a factor inverted by an exchange leaves the scalar 1 / d once it is
             // taken (X diag(1, d) = d diag(1, 1/d) X), for the rest of the launch
             double u_held = 0, i_up = 0, i_down = 0;
             if (best_cost >= mat_cost(u.data(), D)) continue;
-            std::vector<int> to(size_t(M), -1), tob(size_t(M), 0);
-            std::vector<char> inv(size_t(M), 0);
+            Entry d[2] = {kOne, kOne};
+            int to[2] = {-1, -1}, tob[2] = {0, 0};
+            bool inv[2] = {false, false};
             for (int i = 0; i < M; ++i) {
-                const Cx z = u[size_t((1 << i) * D + (1 << i))];
-                if (!usable(z, u)) continue;
+                const Entry& z = u[size_t((1 << i) * D + (1 << i))];
+                if (!usable(z, u) || div_class(z, s) == 1) continue;
                 bool iv = false;
                 int bit = 0;
                 const int p = taker(o, S.R[nth_bit(op.mask, i)], &bit, &iv);
                 if (p < 0) continue;
-                std::vector<Cx> d2 = d;
-                d2[size_t(i)] = exact_div(z, s);
-                if (d2[size_t(i)] == Cx(1, 0)) continue;
-                const std::vector<Cx> v = scaled(u, s, d2);
+                const Entry di = div(z, s);
                 // per amplitude: this op gains, a dense taker may lose
-                double gain = double(best_cost - mat_cost(v.data(), D)) / D;
-                const bool dg = a.ops[p].code == QS_OP_DIAG;
-                if (!dg) {
-                    std::vector<Cx> w = m[size_t(p)];
+                const int cost = rows_cost(u, M, own | (1 << i));
+                double gain = double(best_cost - cost) / D;
+                if (a.ops[p].code != QS_OP_DIAG) {
+                    std::vector<Entry> w = m[size_t(p)];
                     const int D2 = 1 << (ctz(w.size()) / 2);
                     const int before = scaled_cost(w);
-                    take(w, false, index_bit(p, bit), d2[size_t(i)]);
+                    take(w, false, index_bit(p, bit), di);
                     gain -= double(scaled_cost(w) - before) / D2;
                 }
                 if (gain <= 0) continue;
-                d = d2;
-                best = v;
-                best_cost = mat_cost(v.data(), D);
-                to[size_t(i)] = p;
-                tob[size_t(i)] = bit;
-                inv[size_t(i)] = iv;
-                const double ld = std::log2(std::abs(d2[size_t(i)]));
+                own |= 1 << i;
+                best_cost = cost;
+                d[i] = di;
+                to[i] = p;
+                tob[i] = bit;
+                inv[i] = iv;
+                const double ld = log2_abs(di);
                 u_held += std::abs(ld);
                 if (iv) {
                     i_up += std::max(0.0, -ld);
@@ -301,22 +352,22 @@ struct Normaliser {
             down += u_down + i_down;
             held += u_held;
             raised[size_t(o)] += u_up;
-            u = best;
-            total = exact_mul(total, s);
+            u = rows_scaled(u, M, own);
+            total = mul(total, s);
             for (int i = 0; i < M; ++i) {
-                if (to[size_t(i)] < 0) continue;
-                Cx f = d[size_t(i)];
-                if (inv[size_t(i)]) {  // X diag(1, d) = d diag(1, 1/d) X
-                    total = exact_mul(total, f);
-                    raised[size_t(to[size_t(i)])] += std::max(0.0, -std::log2(std::abs(f)));
-                    f = exact_div(Cx(1, 0), f);
+                if (to[i] < 0) continue;
+                Entry f = d[i];
+                if (inv[i]) {  // X diag(1, d) = d diag(1, 1/d) X
+                    total = mul(total, f);
+                    raised[size_t(to[i])] += std::max(0.0, -log2_abs(f));
+                    f = div(kOne, f);
                 }
-                const int p = to[size_t(i)];
-                release[size_t(p)] += std::abs(std::log2(std::abs(d[size_t(i)])));
-                take(m[size_t(p)], a.ops[p].code == QS_OP_DIAG, index_bit(p, tob[size_t(i)]), f);
+                const int p = to[i];
+                release[size_t(p)] += std::abs(log2_abs(d[i]));
+                take(m[size_t(p)], a.ops[p].code == QS_OP_DIAG, index_bit(p, tob[i]), f);
             }
         }
-        if (total == Cx(1, 0)) return;
+        if (total.cl == 1) return;
         // The op that carries the scalars: the amplitudes are low from it until
         // the ops after it have raised them again, by at most max_down.
         int carrier = -1;
@@ -327,8 +378,8 @@ struct Normaliser {
             after += raised[size_t(o)];
             if (low > max_down) break;
             if (controlled(op) || (op.code != QS_OP_MAT && op.code != QS_OP_DIAG)) continue;
-            std::vector<Cx> v = m[size_t(o)];
-            for (Cx& z : v) z = exact_mul(z, total);
+            std::vector<Entry> v = m[size_t(o)];
+            for (Entry& z : v) z.cl = mul_class(z.cl, total.cl);
             double more;
             if (op.code == QS_OP_DIAG) {
                 more = op.nh > 0 ? 0.0 : double(diag_cost(v) - diag_cost(m[size_t(o)])) / double(v.size());
@@ -341,37 +392,46 @@ struct Normaliser {
                 carrier = o;
             }
         }
-        for (Cx& z : m[size_t(carrier)]) z = exact_mul(z, total);
+        for (Entry& z : m[size_t(carrier)]) z = mul(z, total);
     }
-    static int diag_cost(const std::vector<Cx>& v) {
+    static int diag_cost(const std::vector<Entry>& v) {
         int c = 0;
-        for (const Cx& z : v) {
-            const int cl = value_class(z.real(), z.imag());
-            c += cl == 1 ? 0 : cl == 3 ? 4 : 2;
-        }
+        for (const Entry& z : v) c += z.cl == 1 ? 0 : z.cl == 3 ? 4 : 2;
         return c;
     }
     // a factor that is neither zero nor far below the matrix's largest entry
     // (then the matrix keeps its own form)
-    static bool usable(Cx z, const std::vector<Cx>& u) {
-        double top = 0;
-        for (const Cx& e : u) top = std::max(top, std::abs(e));
-        const double r = std::abs(z);
-        return r > top * 0x1p-20 && r >= 0x1p-20 && r <= 0x1p20;
+    static bool usable(const Entry& z, const std::vector<Entry>& u) {
+        long double top = 0;
+        for (const Entry& e : u) top = std::max(top, std::abs(e.z));
+        const long double r = std::abs(z.z);
+        return r > top * 0x1p-20L && r >= 0x1p-20L && r <= 0x1p20L;
     }
-    // rows divided by s times the d_i of the set index bits
-    static std::vector<Cx> scaled(const std::vector<Cx>& u, Cx s, const std::vector<Cx>& d) {
-        const int M = int(d.size()), D = 1 << M;
-        std::vector<Cx> v(u.size());
+    // Row r's factor when the index bits of `own` have theirs taken out: s times
+    // the d_i of r's set bits in `own`, d_i = u_ii / s (so one such bit: u_ii
+    // itself).
+    static Entry row_factor(const std::vector<Entry>& u, int M, int own, int r) {
+        const int D = 1 << M, w = r & own;
+        if (w == 3) return mul(u[size_t(D + 1)], div(u[size_t(2 * D + 2)], u[0]));
+        return u[size_t(w * D + w)];
+    }
+    static int rows_cost(const std::vector<Entry>& u, int M, int own) {
+        const int D = 1 << M;
+        int cost = 0;
         for (int r = 0; r < D; ++r) {
-            Cx f = s;
-            for (int i = 0; i < M; ++i)
-                if ((r >> i) & 1) f = d[size_t(i)] == Cx(1, 0) ? f : exact_mul(f, d[size_t(i)]);
-            for (int c = 0; c < D; ++c) {
-                // the rows whose factor is their own diagonal entry get an exact 1
-                const bool own = c == r && (r == 0 || ((r & (r - 1)) == 0 && !(d[size_t(ctz(size_t(r)))] == Cx(1, 0))));
-                v[size_t(r * D + c)] = own ? Cx(1, 0) : exact_div(u[size_t(r * D + c)], f);
-            }
+            const Entry f = row_factor(u, M, own, r);
+            RowCost row;
+            for (int c = 0; c < D; ++c) row.add(div_class(u[size_t(r * D + c)], f));
+            cost += row.total();
+        }
+        return cost;
+    }
+    static std::vector<Entry> rows_scaled(const std::vector<Entry>& u, int M, int own) {
+        const int D = 1 << M;
+        std::vector<Entry> v(u.size());
+        for (int r = 0; r < D; ++r) {
+            const Entry f = row_factor(u, M, own, r);
+            for (int c = 0; c < D; ++c) v[size_t(r * D + c)] = div(u[size_t(r * D + c)], f);
         }
         return v;
     }
@@ -436,17 +496,31 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
         }
     }
     if (a.nops > 32767) return false;
+    std::vector<uint8_t> ncls(size_t(NM), 3);  // value classes of the entries in the block
     if (!batched && a.nexp == 0) {
-        std::vector<std::vector<Cx>> um(static_cast<size_t>(a.nops));
+        std::vector<std::vector<Entry>> um(static_cast<size_t>(a.nops));
         for (int o = 0; o < a.nops; ++o) {
             const KCopy& c = a.cp[o];
             const int cnt = c.diag ? (1 << c.m) : (1 << (2 * c.m));
-            for (int e = 0; e < cnt; ++e) um[size_t(o)].emplace_back(double(pm[c.soff + e].x), double(pm[c.soff + e].y));
+            long double top = 0;
+            for (int e = 0; e < cnt; ++e) {
+                const V z = pm[c.soff + e];
+                um[size_t(o)].push_back({Cx(z.x, z.y), value_class(z.x, z.y), 0});
+                top = std::max(top, (long double)std::max(std::abs(z.x), std::abs(z.y)));
+            }
+            for (Entry& e : um[size_t(o)]) e.err = 0x1p-53L * top;
         }
         Normaliser(a, um, C128 ? 600.0 : 60.0, C128 ? 300.0 : 24.0).run();
         for (int o = 0; o < a.nops; ++o)
-            for (size_t e = 0; e < um[size_t(o)].size(); ++e)
-                pm[a.cp[o].soff + e] = mk<V>(um[size_t(o)][e].real(), um[size_t(o)][e].imag());
+            for (size_t e = 0; e < um[size_t(o)].size(); ++e) {
+                const Entry& z = um[size_t(o)][e];
+                V& out_z = pm[a.cp[o].soff + e];
+                out_z.x = decltype(out_z.x)(z.z.real());
+                out_z.y = decltype(out_z.y)(z.z.imag());
+                ncls[size_t(a.cp[o].soff) + e] = uint8_t(z.cl);
+            }
+    } else {
+        for (int i = 0; i < NM; ++i) ncls[size_t(i)] = uint8_t(value_class(pm[i].x, pm[i].y));
     }
     // tile position of the psi/lam pair bit (adjoint pair passes)
     int pair_tile = -1;
@@ -509,7 +583,7 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
             scls[size_t(c.soff + e)] = uint8_t(cl);
         }
     }
-    auto vclass = [&](int o, int idx) -> int { return strided[o] ? int(scls[size_t(idx)]) : value_class(pm[idx].x, pm[idx].y); };
+    auto vclass = [&](int o, int idx) -> int { return int((strided[o] ? scls : ncls)[size_t(idx)]); };
     auto mref = [&](int o, int idx) -> std::string {
         return (strided[o] ? "msm[" : "p.m[") + std::to_string(idx) + "]";
     };
