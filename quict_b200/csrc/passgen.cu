@@ -75,20 +75,28 @@ std::string thread_xor_expr(const uint32_t* img, int nT) {
 // diagonal entries of U' are exactly 1 (row r's factor is s times the d_i of
 // its set index bits): an entry 1 costs nothing where a general one costs four
 // instructions per amplitude, a real or imaginary one two.
-//   - s commutes with everything: the launch's scalars are multiplied into one
-//     uncontrolled op (the one whose cost grows least).
+//   - s commutes with everything: the scalars are multiplied into the next
+//     diagonal that is general anyway (at no cost), or those of 8 ops
+//     (complex128: 30) and what is left at the end into the op among them whose
+//     cost grows least.
 //   - D_i moves forward along its bit (through diagonals and controls, across
 //     plain exchanges) into the next uncontrolled op on that bit; d_i = 1 when
 //     no op takes it.
 // The factors are products and quotients in extended precision (64 significand
 // bits), rounded once into the parameter block; a coefficient is never changed
 // by more than that rounding.  Row and scalar factors leave every product's
-// relative rounding error as it is; only the range grows, so the launch's
-// factors are bounded (see run).
-// Which entry becomes 1, and the class of every other one, follows from the
-// classes of the matrices' own entries and from exact equalities between them,
-// never from the size or the last bits of a result: new parameters of a circuit
-// reuse its compiled kernels.
+// relative rounding error as it is; only the range grows.  run() sums the
+// factors' logarithms over the launch, and a launch whose amplitudes could leave
+// the allowed range keeps its own matrices.
+// Which entry becomes 1, the class of every other one and where the scalars go
+// follow from the classes of the matrices' own entries, not from their sizes:
+// new parameters of a circuit reuse its compiled kernels (a limit on the sum of
+// the scalars decided op by op gave 4 to 6 kernels of one complex64 pass in 12
+// parameter sets).  8 ops per carrier: the range holds as long as the scalars
+// average above 2^-7.5, also when a layer repeats one angle; 30-qubit circuit,
+// complex64, 4 / 8 / 16 / all ops of the launch: 2611 / 2570 / 2562 / 2562
+// multiply-adds per amplitude.  complex128, 30 ops: no scalar is below 2^-20, so
+// theirs never exceed the range; 2646, all ops 2646.
 // 30-qubit spread circuit of 1000 gates (B200): 3316 -> 2706 multiply-add
 // instructions per amplitude, complex128 318.3 -> 276.3 ms, complex64 202.4 ->
 // 179.0 ms; 25 qubits, 300 gates, complex64 2.04 -> 1.84 ms, its error against
@@ -194,12 +202,16 @@ int mat_cost(const Entry* m, int D) {  // summed over the rows
 struct Normaliser {
     const RegArgs& a;
     std::vector<std::vector<Entry>>& m;  // per op, slot order (MAT: row-major D x D; DIAG: 2^m entries)
-    // log2 bounds on how far taking factors out may raise (up) and lower (down)
-    // the amplitudes between the launch's load and its store
+    // log2 bounds on how far the factors may raise (up) and lower (down) the
+    // amplitudes between the launch's load and its store; bound on the largest
+    // entry of a matrix and its inverse; ops whose scalars one carrier takes
     const double max_up, max_down;
+    const long double max_entry;
+    const int per_scalar;
 
-    Normaliser(const RegArgs& a_, std::vector<std::vector<Entry>>& m_, double max_up_, double max_down_)
-        : a(a_), m(m_), max_up(max_up_), max_down(max_down_) {}
+    Normaliser(const RegArgs& a_, std::vector<std::vector<Entry>>& m_, bool c128)
+        : a(a_), m(m_), max_up(c128 ? 600 : 60), max_down(c128 ? 300 : 40), max_entry(c128 ? 0x1p700L : 0x1p80L),
+          per_scalar(c128 ? 30 : 8) {}
 
     const KStage& stage_of(int o) const {
         for (int si = 0; si < a.nstages; ++si)
@@ -287,96 +299,47 @@ struct Normaliser {
         return cost;
     }
 
-    // Take factors out of every uncontrolled dense op on one or two bits.
-    void run() {
-        Entry total = kOne;
-        double up = 0, down = 0, held = 0;                 // scalars so far; factors on their way to a taker
-        std::vector<double> raised(size_t(a.nops), 0.0);  // by the scalars that appear at each op
-        std::vector<double> release(size_t(a.nops), 0.0);
+    // Take factors out of every uncontrolled dense op on one or two bits.  False:
+    // the range is exceeded, m is not to be used.
+    bool run() {
+        Entry total = kOne;                                  // scalars taken out and not yet put back
+        std::vector<Entry> late(size_t(a.nops), kOne);       // those that appear at an op
+        std::vector<double> scalar(size_t(a.nops), 0.0);     // log2 changes of the state's scalar, and of what
+        std::vector<double> high(size_t(a.nops), 0.0), low(size_t(a.nops), 0.0);  // factors under way add to it
+        int begin = 0, taken = 0;                            // of the scalars in `total`
+        const auto put_back = [&](int o) {
+            scalar[size_t(o)] += log2_abs(total);
+            for (Entry& z : m[size_t(o)]) z = mul(z, total);
+            total = kOne;
+            begin = o + 1;
+            taken = 0;
+        };
         for (int o = 0; o < a.nops; ++o) {
-            held -= release[size_t(o)];
-            const KOp& op = a.ops[o];
-            if (op.code != QS_OP_MAT || controlled(op)) continue;
-            std::vector<Entry>& u = m[size_t(o)];
-            const int M = popc_c(op.mask), D = 1 << M;
-            if (M > 2) continue;
-            const KStage& S = stage_of(o);
-            const Entry s = u[0];
-            if (!usable(s, u)) continue;
-            int own = 0;  // index bits whose d_i is taken out
-            int best_cost = rows_cost(u, M, own);
-            const double ls = log2_abs(s);
-            const double u_up = std::max(0.0, -ls), u_down = std::max(0.0, ls);
-            // a factor inverted by an exchange leaves the scalar 1 / d once it is
-            // taken (X diag(1, d) = d diag(1, 1/d) X), for the rest of the launch
-            double u_held = 0, i_up = 0, i_down = 0;
-            if (best_cost >= mat_cost(u.data(), D)) continue;
-            Entry d[2] = {kOne, kOne};
-            int to[2] = {-1, -1}, tob[2] = {0, 0};
-            bool inv[2] = {false, false};
-            for (int i = 0; i < M; ++i) {
-                const Entry& z = u[size_t((1 << i) * D + (1 << i))];
-                if (!usable(z, u) || div_class(z, s) == 1) continue;
-                bool iv = false;
-                int bit = 0;
-                const int p = taker(o, S.R[nth_bit(op.mask, i)], &bit, &iv);
-                if (p < 0) continue;
-                const Entry di = div(z, s);
-                // per amplitude: this op gains, a dense taker may lose
-                const int cost = rows_cost(u, M, own | (1 << i));
-                double gain = double(best_cost - cost) / D;
-                if (a.ops[p].code != QS_OP_DIAG) {
-                    std::vector<Entry> w = m[size_t(p)];
-                    const int D2 = 1 << (ctz(w.size()) / 2);
-                    const int before = scaled_cost(w);
-                    take(w, false, index_bit(p, bit), di);
-                    gain -= double(scaled_cost(w) - before) / D2;
-                }
-                if (gain <= 0) continue;
-                own |= 1 << i;
-                best_cost = cost;
-                d[i] = di;
-                to[i] = p;
-                tob[i] = bit;
-                inv[i] = iv;
-                const double ld = log2_abs(di);
-                u_held += std::abs(ld);
-                if (iv) {
-                    i_up += std::max(0.0, -ld);
-                    i_down += std::max(0.0, ld);
-                }
-            }
-            // (written so that a value that is not finite refuses the op)
-            if (!(up + u_up + i_up + held + u_held <= max_up && down + u_down + i_down + held + u_held <= max_down)) continue;
-            up += u_up + i_up;
-            down += u_down + i_down;
-            held += u_held;
-            raised[size_t(o)] += u_up;
-            u = rows_scaled(u, M, own);
-            total = mul(total, s);
-            for (int i = 0; i < M; ++i) {
-                if (to[i] < 0) continue;
-                Entry f = d[i];
-                if (inv[i]) {  // X diag(1, d) = d diag(1, 1/d) X
-                    total = mul(total, f);
-                    raised[size_t(to[i])] += std::max(0.0, -log2_abs(f));
-                    f = div(kOne, f);
-                }
-                const int p = to[i];
-                release[size_t(p)] += std::abs(log2_abs(d[i]));
-                take(m[size_t(p)], a.ops[p].code == QS_OP_DIAG, index_bit(p, tob[i]), f);
-            }
+            total = mul(total, late[size_t(o)]);
+            if (free_diag(o) && total.cl != 1) put_back(o);
+            if (take_out(o, total, late, scalar, high, low) && ++taken == per_scalar) put_back(carrier(begin, o, total));
         }
-        if (total.cl == 1) return;
-        // The op that carries the scalars: the amplitudes are low from it until
-        // the ops after it have raised them again, by at most max_down.
-        int carrier = -1;
-        double least = 1e300, after = 0;
-        for (int o = a.nops - 1; o >= 0; --o) {
+        if (total.cl != 1) put_back(carrier(begin, a.nops - 1, total));
+        double c = 0, h = 0, l = 0;  // the state's scalar; the most and the least that factors under way make of it
+        for (int o = 0; o < a.nops; ++o) {
+            c += scalar[size_t(o)];
+            h += high[size_t(o)];
+            l += low[size_t(o)];
+            // (written so that a value that is not finite is refused)
+            if (!(c + h <= max_up && c + l >= -max_down)) return false;
+            long double top = 0;
+            for (const Entry& z : m[size_t(o)]) top = std::max(top, std::abs(z.z));
+            if (!(top <= max_entry && (top == 0 || top >= 1 / max_entry))) return false;
+        }
+        return true;
+    }
+    // The op of [begin, end] that takes the scalars: the one whose cost grows
+    // least, the last of those.
+    int carrier(int begin, int end, const Entry& total) const {
+        int best = end;
+        double least = 1e300;
+        for (int o = end; o >= begin; --o) {
             const KOp& op = a.ops[o];
-            const double low = after;
-            after += raised[size_t(o)];
-            if (low > max_down) break;
             if (controlled(op) || (op.code != QS_OP_MAT && op.code != QS_OP_DIAG)) continue;
             std::vector<Entry> v = m[size_t(o)];
             for (Entry& z : v) z.cl = mul_class(z.cl, total.cl);
@@ -389,10 +352,74 @@ struct Normaliser {
             }
             if (more < least) {
                 least = more;
-                carrier = o;
+                best = o;
             }
         }
-        for (Entry& z : m[size_t(carrier)]) z = mul(z, total);
+        return best;
+    }
+    // Op o's factors, if taking them out gains.
+    bool take_out(int o, Entry& total, std::vector<Entry>& late, std::vector<double>& scalar, std::vector<double>& high,
+                  std::vector<double>& low) {
+        const KOp& op = a.ops[o];
+        if (op.code != QS_OP_MAT || controlled(op)) return false;
+        std::vector<Entry>& u = m[size_t(o)];
+        const int M = popc_c(op.mask), D = 1 << M;
+        if (M > 2) return false;
+        const KStage& S = stage_of(o);
+        const Entry s = u[0];
+        if (!usable(s, u)) return false;
+        int own = 0;  // index bits whose d_i is taken out
+        int best_cost = rows_cost(u, M, own);
+        if (best_cost >= mat_cost(u.data(), D)) return false;
+        Entry d[2] = {kOne, kOne};
+        int to[2] = {-1, -1}, tob[2] = {0, 0};
+        bool inv[2] = {false, false};
+        for (int i = 0; i < M; ++i) {
+            const Entry& z = u[size_t((1 << i) * D + (1 << i))];
+            if (!usable(z, u) || div_class(z, s) == 1) continue;
+            bool iv = false;
+            int bit = 0;
+            const int p = taker(o, S.R[nth_bit(op.mask, i)], &bit, &iv);
+            if (p < 0) continue;
+            const Entry di = div(z, s);
+            // per amplitude: this op gains, a dense taker may lose
+            const int cost = rows_cost(u, M, own | (1 << i));
+            double gain = double(best_cost - cost) / D;
+            if (a.ops[p].code != QS_OP_DIAG) {
+                std::vector<Entry> w = m[size_t(p)];
+                const int D2 = 1 << (ctz(w.size()) / 2);
+                const int before = scaled_cost(w);
+                take(w, false, index_bit(p, bit), di);
+                gain -= double(scaled_cost(w) - before) / D2;
+            }
+            if (gain <= 0) continue;
+            own |= 1 << i;
+            best_cost = cost;
+            d[i] = di;
+            to[i] = p;
+            tob[i] = bit;
+            inv[i] = iv;
+        }
+        u = rows_scaled(u, M, own);
+        total = mul(total, s);
+        scalar[size_t(o)] -= log2_abs(s);
+        for (int i = 0; i < M; ++i) {
+            if (to[i] < 0) continue;
+            Entry f = d[i];
+            const size_t p = size_t(to[i]);
+            const double ld = log2_abs(f);
+            high[size_t(o)] += std::max(0.0, -ld);
+            high[p] -= std::max(0.0, -ld);
+            low[size_t(o)] += std::min(0.0, -ld);
+            low[p] -= std::min(0.0, -ld);
+            if (inv[i]) {  // X diag(1, d) = d diag(1, 1/d) X: the scalar is there once the factor is taken
+                late[p] = mul(late[p], f);
+                scalar[p] -= ld;
+                f = div(kOne, f);
+            }
+            take(m[p], a.ops[p].code == QS_OP_DIAG, index_bit(to[i], tob[i]), f);
+        }
+        return true;
     }
     static int diag_cost(const std::vector<Entry>& v) {
         int c = 0;
@@ -510,7 +537,8 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
             }
             for (Entry& e : um[size_t(o)]) e.err = 0x1p-53L * top;
         }
-        Normaliser(a, um, C128 ? 600.0 : 60.0, C128 ? 300.0 : 24.0).run();
+        const std::vector<std::vector<Entry>> plain = um;
+        if (!Normaliser(a, um, C128).run()) um = plain;
         for (int o = 0; o < a.nops; ++o)
             for (size_t e = 0; e < um[size_t(o)].size(); ++e) {
                 const Entry& z = um[size_t(o)][e];
