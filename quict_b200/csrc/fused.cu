@@ -509,61 +509,74 @@ std::shared_ptr<const ParamSet> get_params(PlanLaunch& L, int R, const V* hm) {
     return ps;
 }
 
-// Launch the run-time compiled kernel of a planned register pass, if the
-// compiler has it ready (mode SYNC: after compiling it); returns 1 when it
-// was launched, 0 when the generic kernel has to run, < 0 on error.
-template <typename V>
-int launch_jit(V* vec, PlanLaunch& L, int R, const V* hm, const V* mats, double* partials, cudaStream_t st) {
-    const int jm = jit::mode();
-    if (jm == QS_JIT_OFF || hm == nullptr) return 0;
-    const std::shared_ptr<const ParamSet> ps = get_params<V>(L, R, hm);
-    if (!ps) return 0;
-    const JitPass& jp = ps->jp;
-    const RegArgs& args = L.args;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    JitMemo& m = *ps->memo;
+// The run-time compiled kernel of a planned register pass with its parameter
+// block.  fn is null when the compiler does not have it ready (mode SYNC: after
+// compiling it; ASYNC: it is queued from here on) or the pass is not generated.
+struct JitKernel {
+    std::shared_ptr<const ParamSet> ps;
     void* fn = nullptr;
     int occ = 0;
+};
+template <typename V>
+JitKernel jit_kernel(PlanLaunch& L, int R, const V* hm, cudaStream_t st) {
+    JitKernel k;
+    const int jm = jit::mode();
+    int dev = 0;
+    if (jm == QS_JIT_OFF || hm == nullptr || !(k.ps = get_params<V>(L, R, hm))) return k;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        k.ps = nullptr;
+        return k;
+    }
+    JitMemo& m = *k.ps->memo;
     std::string src;
     {
         std::lock_guard<std::mutex> lock(memo_mu());
-        fn = m.fn[dev];
-        occ = m.occ[dev];
-        if (fn == nullptr) src = m.src;
+        k.fn = m.fn[dev];
+        k.occ = m.occ[dev];
+        if (k.fn == nullptr) src = m.src;
     }
-    if (fn == nullptr) {
-        // during stream capture nothing is compiled or loaded: a kernel that is
-        // not loaded yet on this device leaves the pass to the generic kernel
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusActive;
-        const bool capturing = cs != cudaStreamCaptureStatusNone;
-        if (src.empty()) {  // loaded on another device only: regenerate the text
-            JitPass full;
-            if (!gen_pass(&args, R, sizeof(V) == 16, hm, full, true)) return 0;
-            src.swap(full.src);
+    if (k.fn != nullptr) return k;
+    // during stream capture nothing is compiled or loaded: a kernel that is
+    // not loaded yet on this device leaves the pass to the generic kernel
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusActive;
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    if (src.empty()) {  // loaded on another device only: regenerate the text
+        JitPass full;
+        if (!gen_pass(&L.args, R, sizeof(V) == 16, hm, full, true)) {
+            k.ps = nullptr;
+            return k;
         }
-        fn = jit::lookup(src, "qs_pass", jm == QS_JIT_SYNC && !capturing, !capturing, jp.threads, jp.smem, &occ);
-        if (fn != nullptr) {
-            std::lock_guard<std::mutex> lock(memo_mu());
-            m.fn[dev] = fn;
-            m.occ[dev] = occ;
-            std::string().swap(m.src);
-        }
+        src.swap(full.src);
     }
-    if (fn == nullptr) {
+    k.fn = jit::lookup(src, "qs_pass", jm == QS_JIT_SYNC && !capturing, !capturing, k.ps->jp.threads, k.ps->jp.smem, &k.occ);
+    if (k.fn != nullptr) {
+        std::lock_guard<std::mutex> lock(memo_mu());
+        m.fn[dev] = k.fn;
+        m.occ[dev] = k.occ;
+        std::string().swap(m.src);
+    }
+    return k;
+}
+
+// Launch that kernel; returns 1 when it was launched, 0 when the generic kernel
+// has to run, < 0 on error.
+template <typename V>
+int launch_jit(V* vec, PlanLaunch& L, int R, const V* hm, const V* mats, double* partials, cudaStream_t st) {
+    const JitKernel k = jit_kernel<V>(L, R, hm, st);
+    if (!k.ps) return 0;
+    if (k.fn == nullptr) {
         jit::count_launch(false);
         return 0;
     }
-    if (occ < 1) occ = 1;
-    int rc;
-    const uint64_t ntiles = uint64_t(1) << (args.n - args.K);
-    const uint64_t cap = uint64_t(sm_count()) * uint64_t(occ);
+    const JitPass& jp = k.ps->jp;
+    const uint64_t ntiles = uint64_t(1) << (L.args.n - L.args.K);
+    const uint64_t cap = uint64_t(sm_count()) * uint64_t(k.occ < 1 ? 1 : k.occ);
     void* vp = vec;
     const void* mp = mats;
     void* pp = partials;
     void* params[] = {&vp, const_cast<uint64_t*>(jp.params.data()), &mp, &pp};
-    rc = jit::launch(fn, unsigned(ntiles < cap ? ntiles : cap), unsigned(jp.threads), jp.smem, st, params);
+    const int rc = jit::launch(k.fn, unsigned(ntiles < cap ? ntiles : cap), unsigned(jp.threads), jp.smem, st, params);
     if (rc) return rc;
     jit::count_launch(true);
     return 1;
@@ -607,6 +620,9 @@ int launch_reg_k(V* vec, int n, const qs_pass& ps, const qs_op* ops, const V* ma
                 if (jr == 0) break;
             }
             if (done == plan->launches.size()) return QS_OK;
+            // the ones after it do not run now, but are queued with it
+            for (size_t li = done + 1; jit::mode() == QS_JIT_ASYNC && li < plan->launches.size(); ++li)
+                jit_kernel<V>(*plan->launches[li], RJ, hm, st);
             for (int i : plan->launches[done]->rem) rest_ops.push_back(ops[ps.op_begin + i]);
             rest.op_begin = 0;
             rest.op_count = int(rest_ops.size());
