@@ -204,6 +204,9 @@ int qs_jit_wait(double timeout_s);
  * launches of compiled kernels, launches that ran the generic kernel while a
  * compilation was pending, total compile milliseconds, cache hits. */
 int qs_jit_stats(int64_t* out, int n);
+/* Bytes of the plans and parameter blocks of fused passes that are kept between
+ * launches (host memory, 64 MB at most). */
+int64_t qs_plan_store_bytes(void);
 /* Drop queued compilations and wait for the running ones to finish (call
  * before the process exits while compilations may be running; passes not yet
  * compiled keep running on the generic kernels). */

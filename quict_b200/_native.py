@@ -156,6 +156,7 @@ SIGNATURES = {
     "qs_jit_set_mode": (_i, [_i]),
     "qs_jit_wait": (_i, [_d]),
     "qs_jit_stats": (_i, [C.POINTER(C.c_int64), _i]),
+    "qs_plan_store_bytes": (_i64, []),
     "qs_jit_last_log": (C.c_char_p, []),
     "qs_jit_compile_check": (_i, [C.c_char_p, C.POINTER(C.c_int64)]),
     "qs_jit_pass_source": (_i, [_i, _i, C.POINTER(qs_pass), C.POINTER(qs_op), _i64, _vp, _i64, _i, C.c_char_p, _sz,

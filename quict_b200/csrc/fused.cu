@@ -24,7 +24,6 @@
 // (statevector_simulator.py:155-164, gate_function.py:31-1031).
 #include <algorithm>
 #include <array>
-#include <atomic>
 #include <cstdarg>
 #include <cstring>
 #include <memory>
@@ -390,7 +389,8 @@ uint64_t plan_key(const RegArgs& a, int R, size_t vsize, const std::vector<uint8
 // the exact contents of the pass and its ops, and, per plan, the parameter
 // blocks of the matrix values it last ran with (none for per-instance tables,
 // whose values are read on the device).  Contents are compared in full, and the
-// store is dropped whole when it holds more than kPlanBytes.  run() of a known
+// store is dropped whole as soon as plans and parameter blocks together exceed
+// kPlanBytes (plans in use live on with their callers).  run() of a known
 // circuit with the keys of its ops kept as well (B200): 10 qubits, 60 gates
 // 239 -> 81 us; 20 qubits, 200 gates 619 -> 243 us; 25 qubits, 300 gates in
 // complex64 1.84 -> 1.46 ms (the host planned longer than the GPU ran).
@@ -400,8 +400,10 @@ struct ParamSet {
     uint64_t key = 0;                   // plan_key: structure and value classes
     std::shared_ptr<JitMemo> memo;
 };
+struct PassPlan;
 struct PlanLaunch {
     RegArgs args;
+    PassPlan* plan;        // the plan it belongs to
     std::vector<int> rem;  // positions of the pass's ops that had not run before this launch
     std::mutex mu;  // guards sets
     std::vector<std::shared_ptr<const ParamSet>> sets;
@@ -409,13 +411,29 @@ struct PlanLaunch {
 struct PassPlan {
     std::vector<unsigned char> content;
     std::vector<std::unique_ptr<PlanLaunch>> launches;
+    int64_t bytes = 0;    // guarded by g_plan_mu, as is
+    bool stored = false;  // whether g_plans holds it (bytes are then part of g_plan_bytes)
 };
-constexpr size_t kPlanBytes = size_t(64) << 20;
+constexpr int64_t kPlanBytes = int64_t(64) << 20;
 constexpr size_t kParamSets = 8;  // per launch
 
 std::mutex g_plan_mu;  // guards the two below
 std::unordered_map<uint64_t, std::shared_ptr<PassPlan>> g_plans;
-std::atomic<size_t> g_plan_bytes{0};
+int64_t g_plan_bytes = 0;
+
+// Account for a change of a plan's bytes.  With g_plan_mu held.
+void plan_bytes(PassPlan& plan, int64_t change) {
+    plan.bytes += change;
+    if (!plan.stored) return;
+    g_plan_bytes += change;
+    if (g_plan_bytes <= kPlanBytes) return;
+    for (auto& p : g_plans) p.second->stored = false;
+    g_plans.clear();
+    g_plan_bytes = 0;
+}
+int64_t set_bytes(const ParamSet& ps) {
+    return int64_t(sizeof(ParamSet) + ps.values.size() + 8 * ps.jp.params.size() + ps.jp.classes.size());
+}
 
 // Word-wise hash of a byte string (the contents themselves are compared).
 uint64_t hash_bytes(uint64_t h, const void* p, size_t n) {
@@ -453,6 +471,7 @@ std::shared_ptr<PassPlan> get_plan(const qs_pass& ps, const qs_op* ops, int n, i
     while (!rem.empty()) {
         const int next = ps.op_begin + rem.front();
         auto L = std::make_unique<PlanLaunch>();
+        L->plan = plan.get();
         L->rem = rem;
         if (build_reg(ps, ops, rem, n, R, nb, L->args) <= 0) {
             set_error("qs_apply_fused: op %d does not fit a register tile", next);
@@ -461,12 +480,15 @@ std::shared_ptr<PassPlan> get_plan(const qs_pass& ps, const qs_op* ops, int n, i
         plan->launches.push_back(std::move(L));
     }
     std::lock_guard<std::mutex> lock(g_plan_mu);
-    if (g_plan_bytes > kPlanBytes) {
-        g_plans.clear();  // plans in use live on with their callers
-        g_plan_bytes = 0;
+    std::shared_ptr<PassPlan>& slot = g_plans[key];
+    if (slot) {  // the same hash: another thread's plan of this pass, or another pass
+        slot->stored = false;
+        g_plan_bytes -= slot->bytes;
     }
-    g_plan_bytes += content.size() + sizeof(PlanLaunch) * plan->launches.size();
-    g_plans[key] = plan;
+    slot = plan;
+    plan->stored = true;
+    plan_bytes(*plan, int64_t(sizeof(PassPlan) + content.size() +
+                              (sizeof(PlanLaunch) + sizeof(int) * rem.capacity()) * plan->launches.size()));
     return plan;
 }
 
@@ -501,10 +523,17 @@ std::shared_ptr<const ParamSet> get_params(PlanLaunch& L, int R, const V* hm) {
     }
     if (!a.batched) {
         ps->values = values;
-        std::lock_guard<std::mutex> lock(L.mu);
-        if (L.sets.size() >= kParamSets) L.sets.erase(L.sets.begin());
-        else g_plan_bytes += values.size() + 8 * ps->jp.params.size();
-        L.sets.push_back(ps);
+        int64_t change = set_bytes(*ps);
+        {
+            std::lock_guard<std::mutex> lock(L.mu);
+            if (L.sets.size() >= kParamSets) {
+                change -= set_bytes(*L.sets.front());
+                L.sets.erase(L.sets.begin());
+            }
+            L.sets.push_back(ps);
+        }
+        std::lock_guard<std::mutex> lock(g_plan_mu);
+        plan_bytes(*L.plan, change);
     }
     return ps;
 }
@@ -712,6 +741,11 @@ int launch_pass(V* vec, int n, const qs_pass& ps, const qs_op* ops, const V* mat
 }  // namespace qs
 
 using namespace qs;
+
+extern "C" int64_t qs_plan_store_bytes(void) {
+    std::lock_guard<std::mutex> lock(g_plan_mu);
+    return g_plan_bytes;
+}
 
 extern "C" int qs_apply_fused(void* vec, int n, int dtype, const qs_pass* passes, int npasses, const qs_op* ops,
                               int64_t nops_total, const void* mats_dev, int64_t mats_count, void* stream) {
