@@ -12,11 +12,11 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
-#include <complex>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -83,8 +83,9 @@ std::string thread_xor_expr(const uint32_t* img, int nT) {
 //     plain exchanges) into the next uncontrolled op on that bit; d_i = 1 when
 //     no op takes it.
 // The factors are products and quotients in extended precision (64 significand
-// bits), rounded once into the parameter block; a coefficient is never changed
-// by more than that rounding.  Row and scalar factors leave every product's
+// bits), rounded once into the parameter block: a coefficient changes by that
+// rounding, or by its matrix's own where two entries are the same number (see
+// same).  Row and scalar factors leave every product's
 // relative rounding error as it is; only the range grows.  run() sums the
 // factors' logarithms over the launch, and a launch whose amplitudes could leave
 // the allowed range keeps its own matrices.
@@ -94,16 +95,16 @@ std::string thread_xor_expr(const uint32_t* img, int nT) {
 // the scalars decided op by op gave 4 to 6 kernels of one complex64 pass in 12
 // parameter sets).  8 ops per carrier: the range holds as long as the scalars
 // average above 2^-7.5, also when a layer repeats one angle; 30-qubit circuit,
-// complex64, 4 / 8 / 16 / all ops of the launch: 2611 / 2570 / 2562 / 2562
+// complex64, 4 / 8 / 16 / all ops of the launch: 2611 / 2569 / 2561 / 2561
 // multiply-adds per amplitude.  complex128, 30 ops: no scalar is below 2^-20, so
-// theirs never exceed the range; 2646, all ops 2646.
-// 30-qubit spread circuit of 1000 gates (B200): 3316 -> 2706 multiply-add
-// instructions per amplitude, complex128 318.3 -> 276.3 ms, complex64 202.4 ->
-// 179.0 ms; 25 qubits, 300 gates, complex64 2.04 -> 1.84 ms, its error against
-// 64-bit arithmetic 3.8e-7 -> 3.5e-7 (fewer roundings).  Per-instance tables
-// and adjoint passes keep their matrices.
+// theirs never exceed the range; 2638, all ops 2638.
+// 30-qubit spread circuit of 1000 gates at k = 12: 3284 -> 2638 multiply-adds
+// per amplitude in complex128, 3158 -> 2569 in complex64 (B200, when this came
+// in: 318.3 -> 276.3 and 202.4 -> 179.0 ms; now 265.5 and 141.9 ms).  The host
+// takes 20 to 50 us a pass to make a parameter block with or without it.
+// Per-instance tables and adjoint passes keep their matrices.
 #pragma nv_diag_suppress 20208  // long double: host code only here
-using Cx = std::complex<long double>;
+using Ld = long double;
 
 // 0, 1, -1, general (3), real (4), imaginary (5)
 template <typename T>
@@ -114,14 +115,15 @@ int value_class(T x, T y) {
 
 // A matrix entry, its class (what the generated code may assume about it) and
 // the size of the rounding it came with: half a unit in the last place of its
-// matrix's largest entry.
+// matrix's largest component.
 struct Entry {
-    Cx z;
+    Ld re, im;
+    double err;
     int cl;
-    long double err;
+    Ld size() const { return std::max(std::abs(re), std::abs(im)); }
 };
 inline bool is_real(int cl) { return cl == 1 || cl == 2 || cl == 4; }
-const Entry kOne{Cx(1, 0), 1, 0};
+constexpr Entry kOne{1, 0, 0, 1};
 
 int mul_class(int a, int b) {
     if (a == 0 || b == 0) return 0;
@@ -133,49 +135,71 @@ int mul_class(int a, int b) {
 // an entry times a factor
 Entry mul(const Entry& a, const Entry& f) {
     const int cl = mul_class(a.cl, f.cl);
-    const long double x = a.z.real(), y = a.z.imag(), u = f.z.real(), v = f.z.imag();
-    const long double err = a.err == 0 ? 0 : a.err * std::max(std::abs(u), std::abs(v));
-    if (cl == 0) return {Cx(0, 0), 0, err};
-    if (is_real(f.cl)) return {Cx(x * u, y * u), cl, err};
-    if (is_real(a.cl)) return {Cx(x * u, x * v), cl, err};
-    return {Cx(x * u - y * v, x * v + y * u), cl, err};
+    const double err = a.err == 0 ? 0 : a.err * double(f.size());
+    if (cl == 0) return {0, 0, err, 0};
+    if (is_real(f.cl)) return {a.re * f.re, a.im * f.re, err, cl};
+    if (is_real(a.cl)) return {a.re * f.re, a.re * f.im, err, cl};
+    return {a.re * f.re - a.im * f.im, a.re * f.im + a.im * f.re, err, cl};
 }
-// Two entries that are the same number: merged matrices hold such pairs as sums
-// rounded in different orders.  Each component is compared by itself (that of an
-// angle of 2 pi, next to 0, counts), and a pair taken for equal changes its
-// matrix by no more than the roundings it came with.
-bool same(const Entry& a, const Entry& b, const Cx& bz) {
-    const auto near = [e = a.err + b.err](long double x, long double u) {
-        const long double d = std::abs(x - u);
-        return d == 0 || (d <= e && d <= 0x1p-44L * std::abs(u) && x != 0);
-    };
-    return near(a.z.real(), bz.real()) && near(a.z.imag(), bz.imag());
+// Two components that are the same number, or the same up to its sign (-1):
+// merged matrices hold such pairs as sums rounded in different orders.  Each
+// component is compared by itself (that of an angle of 2 pi, next to 0, counts),
+// and a pair taken for equal changes its matrix by no more than the roundings it
+// came with.
+int same(Ld x, Ld u, Ld err) {
+    const Ld d = std::abs(std::abs(x) - std::abs(u));
+    if (!(d == 0 || (d <= err && d <= 0x1p-44L * std::abs(u) && x != 0))) return 0;
+    return (x < 0) == (u < 0) ? 1 : -1;
 }
-// class of a / b: +-1 and +-i where the entries are the same up to that factor
-int div_class(const Entry& a, const Entry& b) {
-    if (a.cl == 0) return 0;
-    if (same(a, b, b.z)) return 1;
-    if (same(a, b, -b.z)) return 2;
-    if (b.cl == 1 || b.cl == 2) return a.cl;
-    if (a.cl == 3 || b.cl == 3) {
-        const Cx t(-b.z.imag(), b.z.real());
-        return same(a, b, t) || same(a, b, -t) ? 5 : 3;
+// i^k with a = i^k b, or -1
+int quarter_turns(const Entry& a, const Entry& b) {
+    const Ld err = Ld(a.err) + Ld(b.err);
+    int r = same(a.re, b.re, err), i = r ? same(a.im, b.im, err) : 0;
+    if (r && i) {
+        if (a.re == 0) return i == 1 ? 0 : 2;
+        if (r == i || a.im == 0) return r == 1 ? 0 : 2;
     }
+    r = same(a.re, b.im, err);
+    i = r ? same(a.im, b.re, err) : 0;
+    if (!r || !i) return -1;
+    if (a.re == 0) return i == 1 ? 1 : 3;  // i times a real number
+    if (a.im == 0) return r == 1 ? 3 : 1;
+    return r != i ? (i == 1 ? 1 : 3) : -1;
+}
+// Class of a / b for two general entries: real or imaginary when they lie on one
+// line through 0, or at a right angle (a row of real numbers times a phase), up
+// to the same roundings; each product of components counts by itself.
+int axis(const Entry& a, const Entry& b) {
+    const Ld err = a.err * b.size() + b.err * a.size();
+    const auto near = [err](Ld p, Ld q) {
+        const Ld d = std::abs(p - q);
+        return d <= err && d <= 0x1p-44L * std::abs(p);
+    };
+    if (near(a.im * b.re, a.re * b.im)) return 4;
+    return near(a.re * b.re, -a.im * b.im) ? 5 : 3;
+}
+// class of a / b
+int div_class(const Entry& a, const Entry& b, int* turns = nullptr) {
+    if (a.cl == 0) return 0;
+    const int t = quarter_turns(a, b);
+    if (turns) *turns = t;
+    if (t >= 0) return t == 0 ? 1 : t == 2 ? 2 : 5;
+    if (b.cl == 1 || b.cl == 2) return a.cl;
+    if (a.cl == 3 && b.cl == 3) return axis(a, b);
+    if (a.cl == 3 || b.cl == 3) return 3;
     return is_real(a.cl) == is_real(b.cl) ? 4 : 5;
 }
-Entry div(const Entry& a, const Entry& b) {
-    const int cl = div_class(a, b);
-    const long double x = a.z.real(), y = a.z.imag(), u = b.z.real(), v = b.z.imag();
-    Cx q(0, 0);
-    if (cl == 1 || cl == 2) q = Cx(cl == 1 ? 1 : -1, 0);
-    else if (cl == 4) q = Cx(is_real(b.cl) ? x / u : y / v, 0);
-    else if (cl == 5 && a.cl == 3) q = Cx(0, same(a, b, Cx(-v, u)) ? 1 : -1);
-    else if (cl == 5) q = Cx(0, is_real(b.cl) ? y / u : -x / v);
-    else if (cl == 3 && is_real(b.cl)) q = Cx(x / u, y / u);
-    else if (cl == 3) q = Cx((x * u + y * v) / (u * u + v * v), (y * u - x * v) / (u * u + v * v));
-    return {q, cl, 0};  // (quotients are factors or final entries)
+Entry div(const Entry& a, const Entry& b) {  // (a factor, or a final entry: err 0)
+    int t = -1;
+    const int cl = div_class(a, b, &t);
+    if (cl == 0) return {0, 0, 0, 0};
+    if (t >= 0) return {Ld(t == 0 ? 1 : t == 2 ? -1 : 0), Ld(t == 1 ? 1 : t == 3 ? -1 : 0), 0, cl};
+    if (is_real(b.cl)) return {a.re / b.re, a.im / b.re, 0, cl};
+    if (b.cl == 5) return {a.im / b.im, -a.re / b.im, 0, cl};
+    const Ld q = 1 / (b.re * b.re + b.im * b.im);
+    return {cl == 5 ? 0 : (a.re * b.re + a.im * b.im) * q, cl == 4 ? 0 : (a.im * b.re - a.re * b.im) * q, 0, cl};
 }
-double log2_abs(const Entry& e) { return double(std::log2(std::abs(e.z))); }
+double log2_abs(const Entry& e) { return 0.5 * std::log2(double(e.re * e.re + e.im * e.im)); }
 
 // Instructions per amplitude of one row: the first term may be a unit entry
 // (taken as is), which the generated code puts first.
@@ -189,40 +213,56 @@ struct RowCost {
     }
     int total() const { return unit ? c - 2 : c; }
 };
-int mat_cost(const Entry* m, int D) {  // summed over the rows
-    int c = 0;
-    for (int r = 0; r < D; ++r) {
-        RowCost row;
-        for (int i = 0; i < D; ++i) row.add(m[r * D + i].cl);
-        c += row.total();
-    }
-    return c;
-}
 
+template <typename V>
 struct Normaliser {
     const RegArgs& a;
-    std::vector<std::vector<Entry>>& m;  // per op, slot order (MAT: row-major D x D; DIAG: 2^m entries)
+    V* const pm;                 // the block's matrices, in slot order
+    std::vector<uint8_t>& ncls;  // and the classes of their entries
     // log2 bounds on how far the factors may raise (up) and lower (down) the
     // amplitudes between the launch's load and its store; bound on the largest
     // entry of a matrix and its inverse; ops whose scalars one carrier takes
-    const double max_up, max_down;
-    const long double max_entry;
-    const int per_scalar;
+    static constexpr bool C128 = sizeof(V) == 16;
+    static constexpr double max_up = C128 ? 600 : 60, max_down = C128 ? 300 : 40;
+    static constexpr Ld max_entry = C128 ? 0x1p700L : 0x1p80L;
+    static constexpr int per_scalar = C128 ? 30 : 8;
 
-    Normaliser(const RegArgs& a_, std::vector<std::vector<Entry>>& m_, bool c128)
-        : a(a_), m(m_), max_up(c128 ? 600 : 60), max_down(c128 ? 300 : 40), max_entry(c128 ? 0x1p700L : 0x1p80L),
-          per_scalar(c128 ? 30 : 8) {}
+    std::unique_ptr<Entry[]> store;
+    std::vector<uint8_t> state;  // per op: 0 not loaded, 1 loaded, 2 changed
+    std::vector<int> stage;      // per op
+    Entry total = kOne;          // scalars taken out and not yet put back
+    std::vector<Entry> late;     // those that appear at an op
+    // log2 changes at each op of the state's scalar, and of the most and the
+    // least that the factors under way make of it
+    std::vector<double> scalar, high, low;
 
-    const KStage& stage_of(int o) const {
+    Normaliser(const RegArgs& a_, V* pm_, std::vector<uint8_t>& ncls_)
+        : a(a_), pm(pm_), ncls(ncls_), store(new Entry[ncls_.size()]), state(size_t(a_.nops), 0),
+          stage(size_t(a_.nops), 0), late(size_t(a_.nops), kOne), scalar(size_t(a_.nops), 0.0),
+          high(size_t(a_.nops), 0.0), low(size_t(a_.nops), 0.0) {
         for (int si = 0; si < a.nstages; ++si)
-            if (o < a.st[si].op_begin + a.st[si].op_count) return a.st[si];
-        return a.st[a.nstages - 1];
+            for (int o = 0; o < a.st[si].op_count; ++o) stage[size_t(a.st[si].op_begin + o)] = si;
+    }
+
+    int count(int o) const { return a.cp[o].diag ? 1 << a.cp[o].m : 1 << (2 * a.cp[o].m); }
+    int dim(int o) const { return 1 << a.cp[o].m; }
+    // op o's matrix (MAT: row-major D x D; DIAG: 2^m entries)
+    Entry* mat(int o) {
+        Entry* const e = store.get() + a.cp[o].soff;
+        if (state[size_t(o)]) return e;
+        state[size_t(o)] = 1;
+        const V* z = pm + a.cp[o].soff;
+        double top = 0;
+        const int cnt = count(o);
+        for (int i = 0; i < cnt; ++i) top = std::max(top, double(std::max(std::abs(z[i].x), std::abs(z[i].y))));
+        for (int i = 0; i < cnt; ++i) e[i] = {z[i].x, z[i].y, 0x1p-53 * top, value_class(z[i].x, z[i].y)};
+        return e;
     }
     static bool controlled(const KOp& op) { return op.scm || op.tctrl || op.gctrl; }
     // index bit of tile bit b among op o's targets, or -1
     int index_bit(int o, int b) const {
         const KOp& op = a.ops[o];
-        const KStage& S = stage_of(o);
+        const KStage& S = a.st[stage[size_t(o)]];
         int i = 0;
         for (int j = 0; j < 6; ++j) {
             if (!((op.mask >> j) & 1)) continue;
@@ -235,17 +275,18 @@ struct Normaliser {
         return -1;
     }
     // a diagonal whose every entry is multiplied anyway takes factors for free
-    bool free_diag(int o) const {
+    bool free_diag(int o) {
         const KOp& op = a.ops[o];
         if (op.code != QS_OP_DIAG || controlled(op)) return false;
         if (op.nh > 0) return true;
-        for (const Entry& z : m[size_t(o)])
-            if (z.cl != 3) return false;
+        const Entry* v = mat(o);
+        for (int i = 0; i < count(o); ++i)
+            if (v[i].cl != 3) return false;
         return true;
     }
     // The op that takes a factor diag(1, d) of tile bit b from op o, the bit it
     // then sits on, and whether an odd number of exchanges inverts it; -1: none.
-    int taker(int o, int b, int* bit, bool* inverted) const {
+    int taker(int o, int b, int* bit, bool* inverted) {
         *inverted = false;
         for (int p = o + 1; p < a.nops; ++p) {
             const KOp& op = a.ops[p];
@@ -259,7 +300,7 @@ struct Normaliser {
                 *inverted = !*inverted;
                 continue;
             } else if (op.code == QS_OP_SWAP) {
-                const KStage& S = stage_of(p);
+                const KStage& S = a.st[stage[size_t(p)]];
                 const int b0 = S.R[nth_bit(op.mask, 0)], b1 = S.R[nth_bit(op.mask, 1)];
                 b = b == b0 ? b1 : b0;
                 continue;
@@ -272,126 +313,153 @@ struct Normaliser {
         return -1;
     }
     // m[p] <- m[p] diag(1, d) on index bit ib (columns; entries of a diagonal)
-    void take(std::vector<Entry>& v, bool diag, int ib, const Entry& d) const {
-        const size_t D = diag ? v.size() : size_t(1) << (ctz(v.size()) / 2);
-        for (size_t e = 0; e < v.size(); ++e)
+    void take(int p, int ib, const Entry& d) {
+        Entry* v = mat(p);
+        state[size_t(p)] = 2;
+        const int D = dim(p);
+        for (int e = 0; e < count(p); ++e)
             if (((e & (D - 1)) >> ib) & 1) v[e] = mul(v[e], d);
     }
-    static int ctz(size_t x) {
-        int c = 0;
-        while (!((x >> c) & 1)) ++c;
-        return c;
-    }
-    // best cost of a matrix whose rows may all be scaled (an estimate)
-    static int scaled_cost(const std::vector<Entry>& v) {
-        const int D = 1 << (ctz(v.size()) / 2);
-        if (D > 4) return mat_cost(v.data(), D);
+    // instructions that a dense op costs more, over its rows, once it has taken
+    // diag(1, d) on index bit ib: as it stands (more than two bits) or with its
+    // rows scaled by their diagonal entries afterwards (an estimate)
+    int take_cost(int p, int ib, const Entry& d) {
+        const Entry* v = mat(p);
+        const int D = dim(p);
         int cost = 0;
         for (int r = 0; r < D; ++r) {
-            const Entry& z = v[size_t(r * D + r)];
-            RowCost row;
+            const Entry z = v[r * D + r], zd = ((r >> ib) & 1) && D <= 4 ? mul(z, d) : z;
+            RowCost before, after;
             for (int c = 0; c < D; ++c) {
-                const Entry& e = v[size_t(r * D + c)];
-                row.add(z.cl == 0 ? e.cl : div_class(e, z));
+                const Entry& e = v[r * D + c];
+                const bool taken = (c >> ib) & 1;
+                if (D > 4 || z.cl == 0) {
+                    before.add(e.cl);
+                    after.add(taken ? mul_class(e.cl, d.cl) : e.cl);
+                } else {
+                    before.add(div_class(e, z));
+                    after.add(div_class(taken ? mul(e, d) : e, zd));
+                }
             }
-            cost += row.total();
+            cost += after.total() - before.total();
         }
         return cost;
     }
 
-    // Take factors out of every uncontrolled dense op on one or two bits.  False:
-    // the range is exceeded, m is not to be used.
+    // Take factors out of every uncontrolled dense op on one or two bits.  False
+    // (and nothing is changed): the range would be exceeded.
     bool run() {
-        Entry total = kOne;                                  // scalars taken out and not yet put back
-        std::vector<Entry> late(size_t(a.nops), kOne);       // those that appear at an op
-        std::vector<double> scalar(size_t(a.nops), 0.0);     // log2 changes of the state's scalar, and of what
-        std::vector<double> high(size_t(a.nops), 0.0), low(size_t(a.nops), 0.0);  // factors under way add to it
-        int begin = 0, taken = 0;                            // of the scalars in `total`
+        int begin = 0, taken = 0;  // of the scalars in `total`
         const auto put_back = [&](int o) {
             scalar[size_t(o)] += log2_abs(total);
-            for (Entry& z : m[size_t(o)]) z = mul(z, total);
+            Entry* v = mat(o);
+            state[size_t(o)] = 2;
+            for (int e = 0; e < count(o); ++e) v[e] = mul(v[e], total);
             total = kOne;
             begin = o + 1;
             taken = 0;
         };
         for (int o = 0; o < a.nops; ++o) {
             total = mul(total, late[size_t(o)]);
-            if (free_diag(o) && total.cl != 1) put_back(o);
-            if (take_out(o, total, late, scalar, high, low) && ++taken == per_scalar) put_back(carrier(begin, o, total));
+            if (total.cl != 1 && free_diag(o)) put_back(o);
+            if (take_out(o) && ++taken == per_scalar) put_back(carrier(begin, o));
         }
-        if (total.cl != 1) put_back(carrier(begin, a.nops - 1, total));
-        double c = 0, h = 0, l = 0;  // the state's scalar; the most and the least that factors under way make of it
+        if (total.cl != 1) put_back(carrier(begin, a.nops - 1));
+        double c = 0, h = 0, l = 0;
         for (int o = 0; o < a.nops; ++o) {
             c += scalar[size_t(o)];
             h += high[size_t(o)];
             l += low[size_t(o)];
             // (written so that a value that is not finite is refused)
             if (!(c + h <= max_up && c + l >= -max_down)) return false;
-            long double top = 0;
-            for (const Entry& z : m[size_t(o)]) top = std::max(top, std::abs(z.z));
+            if (state[size_t(o)] != 2) continue;
+            Ld top = 0;
+            const Entry* v = mat(o);
+            for (int e = 0; e < count(o); ++e) top = std::max(top, v[e].size());
             if (!(top <= max_entry && (top == 0 || top >= 1 / max_entry))) return false;
+        }
+        for (int o = 0; o < a.nops; ++o) {
+            if (state[size_t(o)] != 2) continue;
+            const Entry* v = mat(o);
+            const size_t at = a.cp[o].soff;
+            for (int e = 0; e < count(o); ++e) {
+                pm[at + size_t(e)].x = decltype(V::x)(v[e].re);
+                pm[at + size_t(e)].y = decltype(V::y)(v[e].im);
+                ncls[at + size_t(e)] = uint8_t(v[e].cl);
+            }
         }
         return true;
     }
     // The op of [begin, end] that takes the scalars: the one whose cost grows
     // least, the last of those.
-    int carrier(int begin, int end, const Entry& total) const {
+    int carrier(int begin, int end) {
         int best = end;
         double least = 1e300;
-        for (int o = end; o >= begin; --o) {
+        for (int o = end; o >= begin && least > 0; --o) {
             const KOp& op = a.ops[o];
             if (controlled(op) || (op.code != QS_OP_MAT && op.code != QS_OP_DIAG)) continue;
-            std::vector<Entry> v = m[size_t(o)];
-            for (Entry& z : v) z.cl = mul_class(z.cl, total.cl);
-            double more;
+            const Entry* v = mat(o);
+            const int D = dim(o), cnt = count(o);
+            int more = 0;
             if (op.code == QS_OP_DIAG) {
-                more = op.nh > 0 ? 0.0 : double(diag_cost(v) - diag_cost(m[size_t(o)])) / double(v.size());
+                if (op.nh == 0)
+                    for (int e = 0; e < cnt; ++e) more += diag_cost(mul_class(v[e].cl, total.cl)) - diag_cost(v[e].cl);
             } else {
-                const int D = 1 << (ctz(v.size()) / 2);
-                more = double(mat_cost(v.data(), D) - mat_cost(m[size_t(o)].data(), D)) / D;
+                for (int r = 0; r < D; ++r) {
+                    RowCost before, after;
+                    for (int i = 0; i < D; ++i) {
+                        before.add(v[r * D + i].cl);
+                        after.add(mul_class(v[r * D + i].cl, total.cl));
+                    }
+                    more += after.total() - before.total();
+                }
             }
-            if (more < least) {
-                least = more;
+            if (double(more) / D < least) {
+                least = double(more) / D;
                 best = o;
             }
         }
         return best;
     }
+    static int diag_cost(int cl) { return cl == 1 ? 0 : cl == 3 ? 4 : 2; }
+
     // Op o's factors, if taking them out gains.
-    bool take_out(int o, Entry& total, std::vector<Entry>& late, std::vector<double>& scalar, std::vector<double>& high,
-                  std::vector<double>& low) {
+    bool take_out(int o) {
         const KOp& op = a.ops[o];
-        if (op.code != QS_OP_MAT || controlled(op)) return false;
-        std::vector<Entry>& u = m[size_t(o)];
-        const int M = popc_c(op.mask), D = 1 << M;
-        if (M > 2) return false;
-        const KStage& S = stage_of(o);
+        const int M = a.cp[o].m, D = 1 << M;
+        if (op.code != QS_OP_MAT || controlled(op) || M > 2) return false;
+        Entry* const u = mat(o);
         const Entry s = u[0];
-        if (!usable(s, u)) return false;
+        Ld top = 0;
+        int plain = 0;
+        for (int r = 0; r < D; ++r) {
+            RowCost row;
+            for (int c = 0; c < D; ++c) {
+                top = std::max(top, u[r * D + c].size());
+                row.add(u[r * D + c].cl);
+            }
+            plain += row.total();
+        }
+        if (!usable(s, top)) return false;
         int own = 0;  // index bits whose d_i is taken out
         int best_cost = rows_cost(u, M, own);
-        if (best_cost >= mat_cost(u.data(), D)) return false;
+        if (best_cost >= plain) return false;
         Entry d[2] = {kOne, kOne};
         int to[2] = {-1, -1}, tob[2] = {0, 0};
         bool inv[2] = {false, false};
         for (int i = 0; i < M; ++i) {
-            const Entry& z = u[size_t((1 << i) * D + (1 << i))];
-            if (!usable(z, u) || div_class(z, s) == 1) continue;
+            const Entry& z = u[(1 << i) * D + (1 << i)];
+            if (!usable(z, top)) continue;
+            const Entry di = div(z, s);
+            if (di.cl == 1) continue;
             bool iv = false;
             int bit = 0;
-            const int p = taker(o, S.R[nth_bit(op.mask, i)], &bit, &iv);
+            const int p = taker(o, a.st[stage[size_t(o)]].R[nth_bit(op.mask, i)], &bit, &iv);
             if (p < 0) continue;
-            const Entry di = div(z, s);
             // per amplitude: this op gains, a dense taker may lose
             const int cost = rows_cost(u, M, own | (1 << i));
             double gain = double(best_cost - cost) / D;
-            if (a.ops[p].code != QS_OP_DIAG) {
-                std::vector<Entry> w = m[size_t(p)];
-                const int D2 = 1 << (ctz(w.size()) / 2);
-                const int before = scaled_cost(w);
-                take(w, false, index_bit(p, bit), di);
-                gain -= double(scaled_cost(w) - before) / D2;
-            }
+            if (gain > 0 && a.ops[p].code != QS_OP_DIAG) gain -= double(take_cost(p, index_bit(p, bit), di)) / dim(p);
             if (gain <= 0) continue;
             own |= 1 << i;
             best_cost = cost;
@@ -400,7 +468,8 @@ struct Normaliser {
             tob[i] = bit;
             inv[i] = iv;
         }
-        u = rows_scaled(u, M, own);
+        scale_rows(u, M, own);
+        state[size_t(o)] = 2;
         total = mul(total, s);
         scalar[size_t(o)] -= log2_abs(s);
         for (int i = 0; i < M; ++i) {
@@ -417,50 +486,41 @@ struct Normaliser {
                 scalar[p] -= ld;
                 f = div(kOne, f);
             }
-            take(m[p], a.ops[p].code == QS_OP_DIAG, index_bit(to[i], tob[i]), f);
+            take(to[i], index_bit(to[i], tob[i]), f);
         }
         return true;
     }
-    static int diag_cost(const std::vector<Entry>& v) {
-        int c = 0;
-        for (const Entry& z : v) c += z.cl == 1 ? 0 : z.cl == 3 ? 4 : 2;
-        return c;
-    }
     // a factor that is neither zero nor far below the matrix's largest entry
     // (then the matrix keeps its own form)
-    static bool usable(const Entry& z, const std::vector<Entry>& u) {
-        long double top = 0;
-        for (const Entry& e : u) top = std::max(top, std::abs(e.z));
-        const long double r = std::abs(z.z);
+    static bool usable(const Entry& z, Ld top) {
+        const Ld r = z.size();
         return r > top * 0x1p-20L && r >= 0x1p-20L && r <= 0x1p20L;
     }
     // Row r's factor when the index bits of `own` have theirs taken out: s times
     // the d_i of r's set bits in `own`, d_i = u_ii / s (so one such bit: u_ii
     // itself).
-    static Entry row_factor(const std::vector<Entry>& u, int M, int own, int r) {
+    static Entry row_factor(const Entry* u, int M, int own, int r) {
         const int D = 1 << M, w = r & own;
-        if (w == 3) return mul(u[size_t(D + 1)], div(u[size_t(2 * D + 2)], u[0]));
-        return u[size_t(w * D + w)];
+        if (w == 3) return mul(u[D + 1], div(u[2 * D + 2], u[0]));
+        return u[w * D + w];
     }
-    static int rows_cost(const std::vector<Entry>& u, int M, int own) {
+    static int rows_cost(const Entry* u, int M, int own) {
         const int D = 1 << M;
         int cost = 0;
         for (int r = 0; r < D; ++r) {
             const Entry f = row_factor(u, M, own, r);
             RowCost row;
-            for (int c = 0; c < D; ++c) row.add(div_class(u[size_t(r * D + c)], f));
+            for (int c = 0; c < D; ++c) row.add(div_class(u[r * D + c], f));
             cost += row.total();
         }
         return cost;
     }
-    static std::vector<Entry> rows_scaled(const std::vector<Entry>& u, int M, int own) {
+    static void scale_rows(Entry* u, int M, int own) {
         const int D = 1 << M;
-        std::vector<Entry> v(u.size());
-        for (int r = 0; r < D; ++r) {
-            const Entry f = row_factor(u, M, own, r);
-            for (int c = 0; c < D; ++c) v[size_t(r * D + c)] = div(u[size_t(r * D + c)], f);
-        }
-        return v;
+        Entry f[4];
+        for (int r = 0; r < D; ++r) f[r] = row_factor(u, M, own, r);
+        for (int r = 0; r < D; ++r)
+            for (int c = 0; c < D; ++c) u[r * D + c] = div(u[r * D + c], f[r]);
     }
 };
 
@@ -524,32 +584,8 @@ bool gen_reg_pass(const RegArgs& a, int R, const V* hm, JitPass& out, bool with_
     }
     if (a.nops > 32767) return false;
     std::vector<uint8_t> ncls(size_t(NM), 3);  // value classes of the entries in the block
-    if (!batched && a.nexp == 0) {
-        std::vector<std::vector<Entry>> um(static_cast<size_t>(a.nops));
-        for (int o = 0; o < a.nops; ++o) {
-            const KCopy& c = a.cp[o];
-            const int cnt = c.diag ? (1 << c.m) : (1 << (2 * c.m));
-            long double top = 0;
-            for (int e = 0; e < cnt; ++e) {
-                const V z = pm[c.soff + e];
-                um[size_t(o)].push_back({Cx(z.x, z.y), value_class(z.x, z.y), 0});
-                top = std::max(top, (long double)std::max(std::abs(z.x), std::abs(z.y)));
-            }
-            for (Entry& e : um[size_t(o)]) e.err = 0x1p-53L * top;
-        }
-        const std::vector<std::vector<Entry>> plain = um;
-        if (!Normaliser(a, um, C128).run()) um = plain;
-        for (int o = 0; o < a.nops; ++o)
-            for (size_t e = 0; e < um[size_t(o)].size(); ++e) {
-                const Entry& z = um[size_t(o)][e];
-                V& out_z = pm[a.cp[o].soff + e];
-                out_z.x = decltype(out_z.x)(z.z.real());
-                out_z.y = decltype(out_z.y)(z.z.imag());
-                ncls[size_t(a.cp[o].soff) + e] = uint8_t(z.cl);
-            }
-    } else {
-        for (int i = 0; i < NM; ++i) ncls[size_t(i)] = uint8_t(value_class(pm[i].x, pm[i].y));
-    }
+    for (int i = 0; i < NM; ++i) ncls[size_t(i)] = uint8_t(value_class(pm[i].x, pm[i].y));
+    if (!batched && a.nexp == 0) Normaliser<V>(a, pm, ncls).run();
     // tile position of the psi/lam pair bit (adjoint pair passes)
     int pair_tile = -1;
     for (int b = 0; b < 64 && a.pairmask; ++b)
