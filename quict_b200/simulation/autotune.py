@@ -57,30 +57,31 @@ class Knobs:
 
 def default_knobs(esize: int, n: Optional[int] = None) -> Knobs:
     """Settings used when the cache has no entry: 32-amplitude runs, 2-bit
-    merging, and a tile width by the size of the state.  200 random gates on
-    uniform qubits (B200, device time):
+    merging, and a tile width by type and size.  Random gates on uniform qubits
+    and the spread circuit (B200, device time):
 
-      complex128, k = 10 / 11 / 12: 14 qubits 27 / 27 / 37 us, 18 qubits 37 / 35 /
-        43 us, 22 qubits 222 / 227 / 265 us, 24 qubits 1243 / 976 / 1104 us, 26
-        qubits 4.07 / 3.68 / 3.82 ms, 28 qubits 19.4 / 16.0 / 15.9 ms
-      complex64, k = 11 / 12 / 13: 14 qubits 23 / 24 / 39 us, 18 qubits 29 / 27 / 41
-        us, 20 qubits 45 / 43 us at 11 / 12, 22 qubits 129 / 138 / 162 us, 24
-        qubits 497 / 552 / 459 us, 25 qubits (300 gates) 1316 / 1238 us at 12 / 13,
-        26 qubits 1.92 / 1.91 / 1.92 ms, 28 qubits 8.47 / 8.02 / 8.08 ms; on 400
-        gates of the spread circuit 15.5 / 14.4 / 23.3 ms
+      complex64, 12: time at k = 12 over k = 13, geometric mean of four circuits
+        of 300 gates, 22 / 23 / 24 / 25 / 26 / 27 / 28 qubits: spread 0.67 / 0.67 /
+        0.62 / 0.64 / 0.66 / 0.68 / 0.67, uniform 0.96 / 1.01 / 0.98 / 0.99 / 1.06 /
+        1.03 / 0.96; k = 11 over k = 12, 13 / 14 / 15 / 16 / 17 / 18 / 20 qubits:
+        spread 0.99 / 1.01 / 1.03 / 1.09 / 1.08 / 1.12 / 1.11, uniform 0.99 / 1.02 /
+        1.09 / 1.04 / 0.99 / 1.03 / 1.05
+      complex128, 11 below 27 qubits, 12 from there: k = 11 / 12, 200 gates,
+        spread: 15 qubits 67 / 75 us, 20 qubits 112 / 105 us, 22 qubits 296 / 308
+        us, 25 qubits 2.05 / 2.02 ms, 26 qubits 3.97 / 3.92 ms, 28 qubits 15.6 / 15.4
+        ms; uniform: 50 / 56 us, 105 / 97 us, 265 / 327 us, 2.18 / 2.05 ms, 3.75 / 4.01
+        ms, 18.0 / 17.4 ms (k = 10: 52 us, 105 us, 306 us, 2.35 ms, 4.62 ms, 21.5 ms)
 
-    On a small state narrow tiles give more SMs a tile; a state that fits the
-    L2 cache is read cheaply, so several CTAs per SM are worth more passes; just
-    beyond it a pass saved counts most; on the largest the widest complex64
-    tiles, one CTA per SM, lose more on dense passes than they save.  Without `n` (and for density matrices,
-    whose 12-qubit noisy runs took 2.97 ms at k = 12 and 3.20 ms at k = 11): the
-    widest tiles."""
+    A complex64 tile of 2^12 amplitudes leaves room for several CTAs an SM with
+    16 amplitudes a thread; 2^13 is one CTA with 32, which dense passes pay for.
+    On a small complex128 state narrow tiles give more SMs a tile; on a large one
+    a pass saved counts more.  Without `n` (and for density matrices, whose
+    12-qubit noisy runs took 2.97 ms at k = 12 and 3.20 ms at k = 11): the widest
+    tiles."""
     if n is None:
         k = 12 if esize == 16 else 13
-    elif esize == 16:
-        k = 11 if n < 27 else 12
     else:
-        k = 11 if n < 17 else 13 if 24 <= n < 26 else 12
+        k = 11 if esize == 16 and n < 27 else 12
     return Knobs(k, 5, 2)
 
 
