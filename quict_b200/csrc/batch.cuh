@@ -133,11 +133,17 @@ __device__ void ham_range(V* __restrict__ pl, const BInst& I, const BTerm* __res
     } else {
         for (uint64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
             double re = 0.0, im = 0.0;
-            for (int t = 0; t < I.nterms; ++t) {
-                const uint64_t src = j ^ tm[t].x;
+            int t = 0;
+            while (t < I.nterms) {
+                const uint64_t x = tm[t].x;
+                const uint64_t src = j ^ x;
                 const V a = __ldcg(psi + src);
-                const bool neg = __popcll(tm[t].z & src) & 1;
-                const double sr = neg ? -tm[t].cre : tm[t].cre, si = neg ? -tm[t].cim : tm[t].cim;
+                double sr = 0.0, si = 0.0;
+                for (; t < I.nterms && tm[t].x == x; ++t) {
+                    const bool neg = __popcll(tm[t].z & src) & 1;
+                    sr += neg ? -tm[t].cre : tm[t].cre;
+                    si += neg ? -tm[t].cim : tm[t].cim;
+                }
                 const double ar = double(a.x), ai = double(a.y);
                 re += sr * ar - si * ai;
                 im += sr * ai + si * ar;

@@ -13,9 +13,11 @@ constexpr int kThreads = 256;
 constexpr int kMaxTerms = 128;
 constexpr uint64_t kMaxInnerBlocks = 1024;  // partial sums per instance (workspace: 16 B each)
 
-// Terms in pauli_before order.
+// Terms of one X mask together: group g is the terms [gbeg[g], gbeg[g+1]).
 struct PauliTerms {
-    int n, cplx;
+    int n, cplx, ngroups;
+    int gbeg[kMaxTerms + 1];
+    uint64_t gx[kMaxTerms];                  // per group
     uint64_t xs[kMaxTerms], zs[kMaxTerms];
     double cre[kMaxTerms], cim[kMaxTerms];  // coefficient times i^popc(x & z)
     __device__ __forceinline__ uint64_t x(int t) const { return xs[t]; }
@@ -24,9 +26,9 @@ struct PauliTerms {
     __device__ __forceinline__ double im(int t) const { return cim[t]; }
 };
 
-// out = H psi, eight amplitudes per thread (N >= 2048).  2^24 amplitudes in
-// complex64, 31 terms with 17 X masks (B200): 440 us; 782 us with one parity per
-// term and amplitude.
+// out = H psi, eight amplitudes per thread (terms in pauli_before order).  2^24
+// amplitudes in complex64, 31 terms with 17 X masks (B200): 446 us; 789 us with
+// one parity per term and amplitude.
 template <typename V, bool CPLX>
 __global__ void __launch_bounds__(kThreads)
 k_pauli_sum8(const V* __restrict__ psi, V* __restrict__ out, uint64_t N, const __grid_constant__ PauliTerms p) {
@@ -40,18 +42,23 @@ k_pauli_sum8(const V* __restrict__ psi, V* __restrict__ out, uint64_t N, const _
     }
 }
 
-// The same for vectors below 2048 amplitudes: one amplitude per thread.
+// The same with one amplitude per thread: per group psi[j ^ x] is read once and
+// multiplied by the group's signed coefficient sum (FP64).
 template <typename V>
 __global__ void __launch_bounds__(kThreads)
 k_pauli_sum(const V* __restrict__ psi, V* __restrict__ out, uint64_t N, const __grid_constant__ PauliTerms p) {
     const uint64_t stride = uint64_t(gridDim.x) * kThreads;
     for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < N; j += stride) {
         double re = 0.0, im = 0.0;
-        for (int t = 0; t < p.n; ++t) {
-            const uint64_t src = j ^ p.xs[t];
+        for (int g = 0; g < p.ngroups; ++g) {
+            const uint64_t src = j ^ p.gx[g];
             const V a = psi[src];
-            const bool neg = __popcll(p.zs[t] & src) & 1;
-            const double sr = neg ? -p.cre[t] : p.cre[t], si = neg ? -p.cim[t] : p.cim[t];
+            double sr = 0.0, si = 0.0;
+            for (int t = p.gbeg[g]; t < p.gbeg[g + 1]; ++t) {
+                const bool neg = __popcll(p.zs[t] & src) & 1;
+                sr += neg ? -p.cre[t] : p.cre[t];
+                si += neg ? -p.cim[t] : p.cim[t];
+            }
             const double ar = double(a.x), ai = double(a.y);
             re += sr * ar - si * ai;
             im += sr * ai + si * ar;
@@ -139,8 +146,25 @@ extern "C" int qs_apply_pauli_sum(const void* psi, void* out, int n, int dtype, 
         QS_REQUIRE((xmask[t] >> n) == 0 && (zmask[t] >> n) == 0, "term %d acts on bits >= n", t);
         order[t] = t;
     }
-    std::stable_sort(order, order + nterms,
-                     [&](int a, int b) { return pauli_before(xmask[a], zmask[a], xmask[b], zmask[b]); });
+    std::stable_sort(order, order + nterms, [&](int a, int b) { return xmask[a] < xmask[b]; });
+    p.ngroups = 0;
+    for (int i = 0; i < nterms; ++i)
+        if (i == 0 || xmask[order[i]] != xmask[order[i - 1]]) {
+            p.gx[p.ngroups] = xmask[order[i]];
+            p.gbeg[p.ngroups++] = i;
+        }
+    p.gbeg[p.ngroups] = nterms;
+    const uint64_t N = uint64_t(1) << n;
+    // Eight amplitudes per thread from 2^20 amplitudes on, where the masks are
+    // all different (a transform per term) from 2^22.  Below, an eighth of the
+    // threads do not hide the terms' latency.  31 terms with 17 masks / 128 with
+    // one / 100 with 100, complex64 (B200), one against eight amplitudes: 2^14
+    // 6.3, 18.6 / 6.3, 19.8 / 24, 109 us; 2^18 16.6, 21.1 / 22.7, 20.6 / 64, 121
+    // us; 2^20 54, 41 / 85, 37 / 250, 268 us; 2^22 202, 110 / 323, 94 / 966, 943 us.
+    const bool eight = N >= (uint64_t(1) << (p.ngroups < nterms ? 20 : 22));
+    if (eight)
+        std::stable_sort(order, order + nterms,
+                         [&](int a, int b) { return pauli_before(xmask[a], zmask[a], xmask[b], zmask[b]); });
     p.cplx = 0;
     for (int i = 0; i < nterms; ++i) {
         const int t = order[i];
@@ -157,13 +181,12 @@ extern "C" int qs_apply_pauli_sum(const void* psi, void* out, int n, int dtype, 
         p.cim[i] = im;
         if (im != 0.0) p.cplx = 1;
     }
-    const uint64_t N = uint64_t(1) << n;
     const cudaStream_t st = as_stream(stream);
     auto launch = [&](auto zero) {
         using V = decltype(zero);
         const V* in = static_cast<const V*>(psi);
         V* o = static_cast<V*>(out);
-        if (N < kPauliChunk) {
+        if (!eight) {
             k_pauli_sum<V><<<grid_for(N, kThreads, 8), kThreads, 0, st>>>(in, o, N, p);
             return;
         }

@@ -1,0 +1,55 @@
+"""Both sides of the sizes at which a call changes its kernel: Pauli sums with
+shared and with all different X masks around 2^20 and 2^22 amplitudes, against
+the same sums in torch's FP64 (1e-12 / 1e-5, as state-vector runs)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+TOL = {torch.complex128: 1e-12, torch.complex64: 1e-5}
+
+
+def _state(n, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    v = torch.view_as_complex(torch.randn((1 << n, 2), generator=g, device="cuda", dtype=torch.float64))
+    return (v / torch.linalg.vector_norm(v)).to(dtype)
+
+
+def _qs(dtype):
+    from quict_b200 import _native as N
+    return N.QS_C128 if dtype == torch.complex128 else N.QS_C64
+
+
+def _parity(x):
+    for s in (16, 8, 4, 2, 1):
+        x = x ^ (x >> s)
+    return x & 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.complex128, torch.complex64])
+@pytest.mark.parametrize("masks", ["shared", "different"])
+@pytest.mark.parametrize("n", [11, 19, 20, 21, 22])
+def test_pauli_sums(n, masks, dtype):
+    from quict_b200 import _native as N
+    rng = np.random.default_rng(n)
+    nt = 12
+    x = rng.choice(1 << n, nt, replace=False).astype(np.uint64)
+    if masks == "shared":
+        x[4:] = x[:4].repeat(2)
+    z = rng.integers(0, 1 << n, nt, dtype=np.uint64)
+    c = rng.normal(size=nt)
+    psi = _state(n, dtype)
+    out = torch.full_like(psi, float("nan"))
+    cc = np.ascontiguousarray(np.stack([c, np.zeros(nt)], 1).ravel())
+    N.call("qs_apply_pauli_sum", C.c_void_p(psi.data_ptr()), C.c_void_p(out.data_ptr()), n, _qs(dtype),
+           x.ctypes.data_as(C.c_void_p), z.ctypes.data_as(C.c_void_p), cc.ctypes.data_as(C.c_void_p), nt, None)
+    h = psi.to(torch.complex128)
+    j = torch.arange(1 << n, device="cuda")
+    want = torch.zeros_like(h)
+    for t in range(nt):
+        src = j ^ int(x[t])
+        sign = 1.0 - 2.0 * _parity(src & int(z[t])).double()
+        want += c[t] * (1j ** (int(x[t]) & int(z[t])).bit_count()) * sign * h[src]
+    assert float((out.to(torch.complex128) - want).abs().max()) <= TOL[dtype]
