@@ -500,11 +500,13 @@ k_kq_reg(V* __restrict__ v, uint64_t items, Plan plan, uint64_t cmask, InsertPla
 // shared memory (columns), multiplies them by the matrix, which it reads in
 // tiles of BK columns, and scatters them back.  A thread accumulates TM x TG
 // outputs, rows and columns strided so that the shared-memory reads of a warp
-// are contiguous; the sums run over the matrix columns in order.  Bound by the
-// FP64 / FP32 pipe: 16 outputs per thread and step take 8 shared loads for 64
-// multiply-adds.  Each matrix entry is read once per G groups (one CTA per
-// group, one row per thread and strided matrix reads before: 6-qubit gate on
-// 20 qubits, complex128, 325 us, now 53 us).
+// are contiguous; the sums run over the matrix columns in order: 16 outputs per
+// thread and step take 8 shared loads for 64 multiply-adds.  Each matrix entry is
+// read once per G groups (one CTA per group, one row per thread and strided
+// matrix reads before: 6-qubit gate on 20 qubits, complex128, 325 us, now 53 us).
+// Bound by latency: at 24 qubits (827 us) the FP64 pipe is 30 % active, one CTA
+// of 8 warps an SM (132 registers a thread) waits for each tile of the matrix.
+// With few groups k_kq_one below is faster (see apply_kq_t).
 // The gather walks the target bits and the lowest free bits together in
 // ascending vector order, so global accesses are as contiguous as the bits
 // allow; column G pads the rows against bank conflicts.
@@ -764,6 +766,41 @@ int apply_2q_t(void* vec, int n, int bhi, int blo, uint64_t cmask, int kind, con
     return QS_OK;
 }
 
+// One CTA per group, for as many groups as the SMs take at once: gather 2^k
+// amplitudes into shared memory, each thread makes rows r = tid, tid + blockDim
+// ... .  A group's time is that of one chain of multiply-adds per row; nothing is
+// copied or waited for between columns.
+template <typename V>
+__global__ void __launch_bounds__(256)
+k_kq_one(V* __restrict__ v, uint64_t items, Plan plan, uint64_t cmask, InsertPlan<10> spread, int k,
+         const double2* __restrict__ M) {
+    extern __shared__ unsigned char smem_raw[];
+    V* s = reinterpret_cast<V*>(smem_raw);
+    const int D = 1 << k;
+    for (uint64_t j = blockIdx.x; j < items; j += gridDim.x) {
+        uint64_t base = expand(j, plan) | cmask;
+        __syncthreads();
+        for (int r = threadIdx.x; r < D; r += blockDim.x) {
+            uint64_t o = 0;
+            for (int t = 0; t < k; ++t)
+                if ((r >> (k - 1 - t)) & 1) o |= uint64_t(1) << spread.b[t];
+            s[r] = v[base | o];
+        }
+        __syncthreads();
+        for (int r = threadIdx.x; r < D; r += blockDim.x) {
+            V acc = mk<V>(0.0, 0.0);
+            for (int c = 0; c < D; ++c) {
+                double2 m = M[uint64_t(r) * D + c];
+                acc = cfma(mk<V>(m.x, m.y), s[c], acc);
+            }
+            uint64_t o = 0;
+            for (int t = 0; t < k; ++t)
+                if ((r >> (k - 1 - t)) & 1) o |= uint64_t(1) << spread.b[t];
+            v[base | o] = acc;
+        }
+    }
+}
+
 template <typename V, int K, int G, int THREADS, int TM, int TG, int BK>
 int launch_kq(V* v, int n, const int32_t* bits, uint64_t cmask, uint64_t tmask, const double2* M, cudaStream_t st) {
     constexpr int lg = G == 128 ? 7 : G == 64 ? 6 : G == 32 ? 5 : G == 16 ? 4 : 3;
@@ -816,6 +853,17 @@ int apply_kq_t(void* vec, int n, int k, const int32_t* bits, uint64_t cmask, con
     Plan p = make_plan(cmask | tmask);
     uint64_t items = uint64_t(1) << (n - p.nb);
     const double2* M = static_cast<const double2*>(mat);
+    // One CTA per group while an SM has at most two of them (9 and 10 qubits:
+    // one).  One CTA per group against tiles, complex128 (B200): 128 groups, 6 / 7 /
+    // 8 / 9 / 10 qubits 10, 17 / 17, 25 / 43, 101 / 153, 205 / 585, 806 us; 256
+    // groups 13, 17 / 25, 25 / 80, 103 / 298, 205 / 1156, 808 us; 512 groups 18, 18 /
+    // 44, 26 / 155, 105 us.  complex64 alike (128 groups 11, 15 / 17, 28 / 41, 89 /
+    // 149, 183 / 566, 530 to 590 us); at 5 qubits tiles always (8, 6 us).
+    if (k >= 6 && items <= uint64_t(sm_count()) * (k <= 8 ? 2 : 1)) {
+        k_kq_one<V><<<unsigned(items), 256, sizeof(V) << k, st>>>(v, items, p, cmask, spread, k, M);
+        QS_CHECK_LAUNCH("qs_apply_kq(group)");
+        return QS_OK;
+    }
     switch (k) {
         case 1: k_kq_reg<V, 1><<<grid_for(items, 128, 16), 128, 0, st>>>(v, items, p, cmask, spread, M); break;
         case 2: k_kq_reg<V, 2><<<grid_for(items, 128, 16), 128, 0, st>>>(v, items, p, cmask, spread, M); break;

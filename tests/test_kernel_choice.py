@@ -1,6 +1,8 @@
 """Both sides of the sizes at which a call changes its kernel: Pauli sums with
-shared and with all different X masks around 2^20 and 2^22 amplitudes, against
-the same sums in torch's FP64 (1e-12 / 1e-5, as state-vector runs)."""
+shared and with all different X masks around 2^20 and 2^22 amplitudes, dense
+gates on 6 to 10 qubits with as many groups as the SMs take at once and more;
+against the same sums and products in torch's FP64 (1e-12 / 1e-5, as
+state-vector runs)."""
 import ctypes as C
 
 import numpy as np
@@ -53,3 +55,37 @@ def test_pauli_sums(n, masks, dtype):
         sign = 1.0 - 2.0 * _parity(src & int(z[t])).double()
         want += c[t] * (1j ** (int(x[t]) & int(z[t])).bit_count()) * sign * h[src]
     assert float((out.to(torch.complex128) - want).abs().max()) <= TOL[dtype]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.complex128, torch.complex64])
+@pytest.mark.parametrize("controls", [0, 1])
+@pytest.mark.parametrize("k", [6, 7, 8, 9, 10])
+def test_dense_gates(k, controls, dtype):
+    from quict_b200.simulation.engine import Engine, require_cuda
+    from quict_b200.simulation.lowering import Op
+    from quict_b200.workloads import haar_unitary
+    rng = np.random.default_rng(k)
+    eng = Engine(require_cuda(0))
+    mat = haar_unitary(rng, 1 << k)
+    for groups in (0, 3, 6, 7, 8, 9, 10):
+        n = k + groups + controls
+        if n > 18:
+            continue
+        bits = [int(b) for b in rng.permutation(n)[:k + controls]]
+        tbits, cbits = bits[:k], tuple(bits[k:])
+        psi = _state(n, dtype)
+        h = psi.to(torch.complex128)
+        idx = torch.arange(1 << n, device="cuda")
+        zero = torch.ones_like(idx, dtype=torch.bool)
+        for b in tbits:
+            zero &= ((idx >> b) & 1) == 0
+        for b in cbits:
+            zero &= ((idx >> b) & 1) == 1
+        spread = torch.tensor([sum(((r >> (k - 1 - j)) & 1) << b for j, b in enumerate(tbits)) for r in range(1 << k)],
+                              device="cuda")
+        cols = idx[zero][None, :] + spread[:, None]
+        want = h.clone()
+        want[cols] = torch.from_numpy(mat).cuda() @ h[cols]
+        eng.apply_single(psi, n, Op("mat", tuple(tbits), cbits, mat))
+        assert float((psi.to(torch.complex128) - want).abs().max()) <= TOL[dtype], (groups, tbits, cbits)
