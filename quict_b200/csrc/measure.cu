@@ -81,10 +81,27 @@ __global__ void __launch_bounds__(kThreads) k_finish(const double* __restrict__ 
     if (threadIdx.x == 0) *out = acc;
 }
 
-// Both walk the pairs of `bit`, four in flight per thread, and read only the
+// Collapse, amplitude by amplitude in vector order: every access of a warp is
+// contiguous.
+template <typename V>
+__global__ void __launch_bounds__(kThreads)
+k_collapse_each(V* __restrict__ v, uint64_t N, int bit, int outcome, double scale) {
+    const uint64_t stride = uint64_t(gridDim.x) * kThreads;
+    for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < N; i += stride) {
+        if (int((i >> bit) & 1) == outcome) {
+            V a = v[i];
+            a.x *= scale; a.y *= scale;
+            v[i] = a;
+        } else {
+            v[i] = mk<V>(0.0, 0.0);
+        }
+    }
+}
+
+// The two below walk the pairs of `bit`, U in flight per thread, and read only the
 // half that is kept: 25 qubits in complex64 (B200), 256 MB: collapse 65-88 us
-// (65-95 us when every amplitude was visited one at a time), reset 67 us (131
-// us with a division per component).
+// (65-95 us amplitude by amplitude), reset 67 us (131 us with a division per
+// component).
 template <typename V>
 __global__ void __launch_bounds__(kThreads) k_collapse(V* __restrict__ v, uint64_t items, int bit, int outcome, double scale) {
     constexpr int U = 4;
@@ -121,9 +138,8 @@ __device__ __forceinline__ float div_by(float x, double alpha, double r) {
 
 // Reference reset rule: alpha = sqrt(P0); alpha < 1e-6 -> v0 <- v1, else
 // v0 <- v0 / alpha; v1 <- 0 either way.
-template <typename V>
+template <typename V, int U>
 __global__ void __launch_bounds__(kThreads) k_reset(V* __restrict__ v, uint64_t items, int bit, double alpha, bool move) {
-    constexpr int U = 4;
     const uint64_t stride = uint64_t(gridDim.x) * kThreads, off = uint64_t(1) << bit;
     const double r = 1.0 / alpha;
     for (uint64_t j0 = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j0 < items; j0 += U * stride) {
@@ -457,7 +473,14 @@ extern "C" int qs_collapse(void* vec, int n, int dtype, int bit, int outcome, do
     QS_REQUIRE(outcome == 0 || outcome == 1, "outcome must be 0 or 1");
     uint64_t items = uint64_t(1) << (n - 1);
     unsigned grid = grid_for(items, kThreads * 4, 8);
-    if (dtype == QS_C128) k_collapse<double2><<<grid, kThreads, 0, as_stream(stream)>>>((double2*)vec, items, bit, outcome, scale);
+    // Pairs for complex64 states beyond the L2's reach (2^23 amplitudes): 24 qubits
+    // 39 - 49 us against 41 - 54 us (B200); below, and in complex128, the walk in
+    // vector order is as fast or faster (20 qubits complex64 4.2 against 5.0 us; 26
+    // qubits complex128, bit 0, 343 against 367 us, 24 qubits, bit 23, 70 against 75 us).
+    const uint64_t N = 2 * items;
+    const unsigned each = grid_for(N, kThreads * 4, 8);
+    if (dtype == QS_C128) k_collapse_each<double2><<<each, kThreads, 0, as_stream(stream)>>>((double2*)vec, N, bit, outcome, scale);
+    else if (n < 23)      k_collapse_each<float2><<<each, kThreads, 0, as_stream(stream)>>>((float2*)vec, N, bit, outcome, scale);
     else                  k_collapse<float2><<<grid, kThreads, 0, as_stream(stream)>>>((float2*)vec, items, bit, outcome, scale);
     QS_CHECK_LAUNCH("qs_collapse");
     return QS_OK;
@@ -471,8 +494,11 @@ extern "C" int qs_reset(void* vec, int n, int dtype, int bit, double p0, void* s
     bool move = alpha < 1e-6;
     uint64_t items = uint64_t(1) << (n - 1);
     unsigned grid = grid_for(items, kThreads * 4, 8);
-    if (dtype == QS_C128) k_reset<double2><<<grid, kThreads, 0, as_stream(stream)>>>((double2*)vec, items, bit, alpha, move);
-    else                  k_reset<float2><<<grid, kThreads, 0, as_stream(stream)>>>((float2*)vec, items, bit, alpha, move);
+    // Bits 0 and 1 of complex64, whose pairs share a 32-byte sector: one pair in
+    // flight (26 qubits, B200: 170 us, four 190 us).
+    if (dtype == QS_C128) k_reset<double2, 4><<<grid, kThreads, 0, as_stream(stream)>>>((double2*)vec, items, bit, alpha, move);
+    else if (bit < 2)     k_reset<float2, 1><<<grid, kThreads, 0, as_stream(stream)>>>((float2*)vec, items, bit, alpha, move);
+    else                  k_reset<float2, 4><<<grid, kThreads, 0, as_stream(stream)>>>((float2*)vec, items, bit, alpha, move);
     QS_CHECK_LAUNCH("qs_reset");
     return QS_OK;
 }

@@ -1,8 +1,10 @@
 """Both sides of the sizes at which a call changes its kernel: Pauli sums with
 shared and with all different X masks around 2^20 and 2^22 amplitudes, dense
-gates on 6 to 10 qubits with as many groups as the SMs take at once and more;
-against the same sums and products in torch's FP64 (1e-12 / 1e-5, as
-state-vector runs)."""
+gates on 6 to 10 qubits with as many groups as the SMs take at once and twice
+that, collapse and reset on low and high bits around 2^23 amplitudes; against
+the same rules in torch's FP64.  Tolerances: sums and matrix products as
+state-vector runs (1e-12 / 1e-5), collapse and reset one rounding of each kept
+component."""
 import ctypes as C
 
 import numpy as np
@@ -89,3 +91,29 @@ def test_dense_gates(k, controls, dtype):
         want[cols] = torch.from_numpy(mat).cuda() @ h[cols]
         eng.apply_single(psi, n, Op("mat", tuple(tbits), cbits, mat))
         assert float((psi.to(torch.complex128) - want).abs().max()) <= TOL[dtype], (groups, tbits, cbits)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.complex128, torch.complex64])
+@pytest.mark.parametrize("n", [3, 13, 22, 23, 24])
+def test_collapse_and_reset(n, dtype):
+    from quict_b200.simulation.engine import Engine, require_cuda
+    eng = Engine(require_cuda(0))
+    base = _state(n, dtype)
+    h = base.to(torch.complex128)
+    idx = torch.arange(1 << n, device="cuda")
+    eps = 2.0 ** -52 if dtype == torch.complex128 else 2.0 ** -23
+    for bit in sorted({0, 1, 2, n // 2, n - 1}):
+        one = ((idx >> bit) & 1) == 1
+        for outcome in (0, 1):
+            got = base.clone()
+            eng.collapse(got, n, bit, outcome, 1.25)
+            want = torch.where(one == bool(outcome), h * 1.25, 0)
+            assert bool(((got.to(torch.complex128) - want).abs() <= eps * want.abs()).all())
+        for p in (0.37, 0.0):
+            got = base.clone()
+            eng.reset(got, n, bit, p)
+            want = torch.zeros_like(h)
+            a = float(np.sqrt(p))
+            want[~one] = h[one] if p == 0.0 else torch.complex(h[~one].real / a, h[~one].imag / a)
+            assert bool(((got.to(torch.complex128) - want).abs() <= eps * want.abs()).all())
