@@ -614,8 +614,8 @@ int launch_jit(V* vec, PlanLaunch& L, int R, const V* hm, const V* mats, double*
 // Register bits per thread of generated passes.  complex128: 4, as the generic
 // kernel.  complex64: 4 where a tile of 2^k amplitudes then has at most 256
 // threads (k <= 12), else the generic kernel's 5.  Half the amplitudes per
-// thread leave registers for three times the warps, and passes of complex64 are
-// bound by the issue of dependent instructions, not by their relayouts.  4
+// thread leave registers for three times the warps: three CTAs of 256 threads an
+// SM issue 3.0 instructions a cycle (of 4), the FMA pipe 52 - 55 % active.  4
 // against 5 (B200, k = 12): 30-qubit spread circuit of 1000 gates 147.6 against
 // 163.2 ms (139.2 at nlow = 5), 28 qubits, 400 gates 14.4 against 15.6 ms, 24
 // qubits 643 against 845 us, 18 qubits 27 against 37 us.  QS_JIT_REG_BITS (4 or

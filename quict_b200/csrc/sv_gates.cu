@@ -10,6 +10,7 @@
 //   2q dense / swap        : quads (swap touches only |01>, |10>)
 // Reference kernels replaced: QuICT/ops/gate_kernel/gate_function.py:31-1031.
 #include "common.cuh"
+#include "kq_tiles.h"
 
 namespace qs {
 
@@ -495,109 +496,39 @@ k_kq_reg(V* __restrict__ v, uint64_t items, Plan plan, uint64_t cmask, InsertPla
     }
 }
 
-// -------------------------------------------------- k-qubit dense, 5<=K<=10
-// The gate as a matrix product: a CTA gathers G groups of 2^K amplitudes into
-// shared memory (columns), multiplies them by the matrix, which it reads in
-// tiles of BK columns, and scatters them back.  A thread accumulates TM x TG
-// outputs, rows and columns strided so that the shared-memory reads of a warp
-// are contiguous; the sums run over the matrix columns in order: 16 outputs per
-// thread and step take 8 shared loads for 64 multiply-adds.  Each matrix entry is
-// read once per G groups (one CTA per group, one row per thread and strided
-// matrix reads before: 6-qubit gate on 20 qubits, complex128, 325 us, now 53 us).
-// Bound by latency: at 24 qubits (827 us) the FP64 pipe is 30 % active, one CTA
-// of 8 warps an SM (132 registers a thread) waits for each tile of the matrix.
-// With few groups k_kq_one below is faster (see apply_kq_t).
-// The gather walks the target bits and the lowest free bits together in
-// ascending vector order, so global accesses are as contiguous as the bits
-// allow; column G pads the rows against bank conflicts.
-struct KqMap {
-    int nbits, gbits;      // bits of a tile; of them group bits
-    uint8_t pos[20];       // vector bit, ascending
-    int32_t at[20];        // its step in the shared tile
-};
-
-template <typename V, int K, int G, int THREADS, int TM, int TG, int BK>
-__global__ void __launch_bounds__(THREADS)
-k_kq_tile(V* __restrict__ v, uint64_t tiles, Plan plan, uint64_t cmask, const __grid_constant__ KqMap map,
-          const double2* __restrict__ M) {
-    constexpr int D = 1 << K, GP = G + 1, DP = D + 1;
-    constexpr int RT = D / TM, CT = G / TG;
-    static_assert(RT * CT == THREADS, "one thread per TM x TG outputs");
-    constexpr int LT = THREADS == 512 ? 9 : THREADS == 256 ? 8 : 7;
-    static_assert((1 << LT) == THREADS, "threads");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    V* X = reinterpret_cast<V*>(smem_raw);  // [D][GP]
-    V* A = X + D * GP;                      // [BK][DP]
-    const int tid = threadIdx.x, tx = tid % CT, ty = tid / CT;
-    uint64_t toff = 0;
-    int tat = 0;
-    for (int i = 0; i < LT && i < map.nbits; ++i)
-        if ((tid >> i) & 1) {
-            toff |= uint64_t(1) << map.pos[i];
-            tat += map.at[i];
-        }
-    const int steps = map.nbits > LT ? 1 << (map.nbits - LT) : 1;
-    const bool moves = map.nbits >= LT || tid < (1 << map.nbits);
-    auto part = [&](int i, uint64_t& off, int& at) {
-        off = toff;
-        at = tat;
-        for (int b = 0; b < map.nbits - LT; ++b)
-            if ((i >> b) & 1) {
-                off |= uint64_t(1) << map.pos[LT + b];
-                at += map.at[LT + b];
-            }
-    };
-    if ((1 << map.gbits) < G)  // fewer groups than columns: the others stay 0
-        for (int i = tid; i < D * GP; i += THREADS) X[i] = mk<V>(0.0, 0.0);
-    for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const uint64_t base = expand(t << map.gbits, plan) | cmask;
+// -------------------------------------------------- k-qubit dense, 6<=K<=10, few groups
+// One CTA per group, for as many groups as the SMs take at once: gather 2^k
+// amplitudes into shared memory, each thread makes rows r = tid, tid + blockDim
+// ... .  A group's time is that of one chain of multiply-adds per row; nothing is
+// copied or waited for between columns.
+template <typename V>
+__global__ void __launch_bounds__(256)
+k_kq_one(V* __restrict__ v, uint64_t items, Plan plan, uint64_t cmask, InsertPlan<10> spread, int k,
+         const double2* __restrict__ M) {
+    extern __shared__ unsigned char smem_raw[];
+    V* s = reinterpret_cast<V*>(smem_raw);
+    const int D = 1 << k;
+    for (uint64_t j = blockIdx.x; j < items; j += gridDim.x) {
+        uint64_t base = expand(j, plan) | cmask;
         __syncthreads();
-        if (moves)
-            for (int i = 0; i < steps; ++i) {
-                uint64_t off;
-                int at;
-                part(i, off, at);
-                X[at] = v[base | off];
-            }
-        V acc[TM][TG];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TG; ++j) acc[i][j] = mk<V>(0.0, 0.0);
-        for (int c0 = 0; c0 < D; c0 += BK) {
-            __syncthreads();
-            for (int e = tid; e < D * BK; e += THREADS) {
-                const int r = e / BK, c = e % BK;
-                const double2 m = __ldg(&M[r * D + c0 + c]);
-                A[c * DP + r] = mk<V>(m.x, m.y);
-            }
-            __syncthreads();
-#pragma unroll
-            for (int c = 0; c < BK; ++c) {
-                V a[TM], x[TG];
-#pragma unroll
-                for (int i = 0; i < TM; ++i) a[i] = A[c * DP + i * RT + ty];
-#pragma unroll
-                for (int j = 0; j < TG; ++j) x[j] = X[(c0 + c) * GP + j * CT + tx];
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < TG; ++j) acc[i][j] = cfma(a[i], x[j], acc[i][j]);
-            }
+        for (int r = threadIdx.x; r < D; r += blockDim.x) {
+            uint64_t o = 0;
+            for (int t = 0; t < k; ++t)
+                if ((r >> (k - 1 - t)) & 1) o |= uint64_t(1) << spread.b[t];
+            s[r] = v[base | o];
         }
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TG; ++j) X[(i * RT + ty) * GP + j * CT + tx] = acc[i][j];
-        __syncthreads();
-        if (moves)
-            for (int i = 0; i < steps; ++i) {
-                uint64_t off;
-                int at;
-                part(i, off, at);
-                v[base | off] = X[at];
+        for (int r = threadIdx.x; r < D; r += blockDim.x) {
+            V acc = mk<V>(0.0, 0.0);
+            for (int c = 0; c < D; ++c) {
+                double2 m = M[uint64_t(r) * D + c];
+                acc = cfma(mk<V>(m.x, m.y), s[c], acc);
             }
+            uint64_t o = 0;
+            for (int t = 0; t < k; ++t)
+                if ((r >> (k - 1 - t)) & 1) o |= uint64_t(1) << spread.b[t];
+            v[base | o] = acc;
+        }
     }
 }
 
@@ -766,83 +697,6 @@ int apply_2q_t(void* vec, int n, int bhi, int blo, uint64_t cmask, int kind, con
     return QS_OK;
 }
 
-// One CTA per group, for as many groups as the SMs take at once: gather 2^k
-// amplitudes into shared memory, each thread makes rows r = tid, tid + blockDim
-// ... .  A group's time is that of one chain of multiply-adds per row; nothing is
-// copied or waited for between columns.
-template <typename V>
-__global__ void __launch_bounds__(256)
-k_kq_one(V* __restrict__ v, uint64_t items, Plan plan, uint64_t cmask, InsertPlan<10> spread, int k,
-         const double2* __restrict__ M) {
-    extern __shared__ unsigned char smem_raw[];
-    V* s = reinterpret_cast<V*>(smem_raw);
-    const int D = 1 << k;
-    for (uint64_t j = blockIdx.x; j < items; j += gridDim.x) {
-        uint64_t base = expand(j, plan) | cmask;
-        __syncthreads();
-        for (int r = threadIdx.x; r < D; r += blockDim.x) {
-            uint64_t o = 0;
-            for (int t = 0; t < k; ++t)
-                if ((r >> (k - 1 - t)) & 1) o |= uint64_t(1) << spread.b[t];
-            s[r] = v[base | o];
-        }
-        __syncthreads();
-        for (int r = threadIdx.x; r < D; r += blockDim.x) {
-            V acc = mk<V>(0.0, 0.0);
-            for (int c = 0; c < D; ++c) {
-                double2 m = M[uint64_t(r) * D + c];
-                acc = cfma(mk<V>(m.x, m.y), s[c], acc);
-            }
-            uint64_t o = 0;
-            for (int t = 0; t < k; ++t)
-                if ((r >> (k - 1 - t)) & 1) o |= uint64_t(1) << spread.b[t];
-            v[base | o] = acc;
-        }
-    }
-}
-
-template <typename V, int K, int G, int THREADS, int TM, int TG, int BK>
-int launch_kq(V* v, int n, const int32_t* bits, uint64_t cmask, uint64_t tmask, const double2* M, cudaStream_t st) {
-    constexpr int lg = G == 128 ? 7 : G == 64 ? 6 : G == 32 ? 5 : G == 16 ? 4 : 3;
-    static_assert((1 << lg) == G, "G");
-    const uint64_t fixed = cmask | tmask;
-    const int free_bits = n - __builtin_popcountll(fixed);
-    // Fewer wide tiles than SMs: narrow tiles of 8 columns spread the groups
-    // over more SMs, at more matrix reads per group.
-    if constexpr (G > 8)
-        if ((uint64_t(1) << free_bits) / G < uint64_t(sm_count()))
-            return launch_kq<V, K, 8, 128, (1 << K) / 16, 1, 8>(v, n, bits, cmask, tmask, M, st);
-    KqMap map{};
-    map.gbits = lg < free_bits ? lg : free_bits;
-    int g = 0;
-    for (int b = 0; b < n; ++b) {
-        int step = -1;
-        if ((tmask >> b) & 1) {
-            for (int t = 0; t < K; ++t)
-                if (bits[t] == b) step = (1 << (K - 1 - t)) * (G + 1);
-        } else if (!((cmask >> b) & 1) && g < map.gbits) {
-            step = 1 << g++;
-        }
-        if (step < 0) continue;
-        map.pos[map.nbits] = uint8_t(b);
-        map.at[map.nbits++] = step;
-    }
-    const Plan p = make_plan(fixed);
-    const uint64_t tiles = uint64_t(1) << (free_bits - map.gbits);
-    const size_t smem = sizeof(V) * (size_t(1 << K) * (G + 1) + size_t(BK) * ((1 << K) + 1));
-    auto* fn = k_kq_tile<V, K, G, THREADS, TM, TG, BK>;
-    // per call: the attribute belongs to the device, and costs nothing beside the launch
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    if (e != cudaSuccess) {
-        set_error("qs_apply_kq: %s", cudaGetErrorString(e));
-        return QS_ECUDA;
-    }
-    fn<<<grid_for(tiles, 1, smem > 110 * 1024 ? 1 : smem > 72 * 1024 ? 2 : 3), THREADS, smem, st>>>(v, tiles, p, cmask,
-                                                                                                    map, M);
-    QS_CHECK_LAUNCH("qs_apply_kq(tile)");
-    return QS_OK;
-}
-
 template <typename R>
 int apply_kq_t(void* vec, int n, int k, const int32_t* bits, uint64_t cmask, const void* mat, cudaStream_t st) {
     using V = typename CT<R>::V;
@@ -869,12 +723,7 @@ int apply_kq_t(void* vec, int n, int k, const int32_t* bits, uint64_t cmask, con
         case 2: k_kq_reg<V, 2><<<grid_for(items, 128, 16), 128, 0, st>>>(v, items, p, cmask, spread, M); break;
         case 3: k_kq_reg<V, 3><<<grid_for(items, 128, 16), 128, 0, st>>>(v, items, p, cmask, spread, M); break;
         case 4: k_kq_reg<V, 4><<<grid_for(items, 128, 16), 128, 0, st>>>(v, items, p, cmask, spread, M); break;
-        case 5: return launch_kq<V, 5, 128, 256, 4, 4, 8>(v, n, bits, cmask, tmask, M, st);
-        case 6: return launch_kq<V, 6, 64, 256, 4, 4, 8>(v, n, bits, cmask, tmask, M, st);
-        case 7: return launch_kq<V, 7, 32, 256, 4, 4, 8>(v, n, bits, cmask, tmask, M, st);
-        case 8: return launch_kq<V, 8, 16, 256, 4, 4, 8>(v, n, bits, cmask, tmask, M, st);
-        case 9: return launch_kq<V, 9, 8, 256, 8, 2, 4>(v, n, bits, cmask, tmask, M, st);
-        default: return launch_kq<V, 10, 8, 512, 8, 2, 4>(v, n, bits, cmask, tmask, M, st);
+        default: return apply_kq_tiles(sizeof(V) == 16 ? QS_C128 : QS_C64, v, n, k, bits, cmask, tmask, M, st);
     }
     QS_CHECK_LAUNCH("qs_apply_kq");
     return QS_OK;
