@@ -95,12 +95,12 @@ std::string thread_xor_expr(const uint32_t* img, int nT) {
 // the scalars decided op by op gave 4 to 6 kernels of one complex64 pass in 12
 // parameter sets).  8 ops per carrier: the range holds as long as the scalars
 // average above 2^-7.5, also when a layer repeats one angle; 30-qubit circuit,
-// complex64, 4 / 8 / 16 / all ops of the launch: 2611 / 2569 / 2561 / 2561
+// complex64, 4 / 8 / 16 / all ops of the launch: 2582 / 2557 / 2552 / 2552
 // multiply-adds per amplitude.  complex128, 30 ops: no scalar is below 2^-20, so
-// theirs never exceed the range; 2638, all ops 2638.
-// 30-qubit spread circuit of 1000 gates at k = 12: 3284 -> 2638 multiply-adds
-// per amplitude in complex128, 3158 -> 2569 in complex64 (B200, when this came
-// in: 318.3 -> 276.3 and 202.4 -> 179.0 ms; now 265.5 and 141.9 ms).  The host
+// theirs never exceed the range; 2630, all ops 2630.
+// 30-qubit spread circuit of 1000 gates at k = 12: 3284 -> 2630 multiply-adds
+// per amplitude in complex128, 3158 -> 2557 in complex64 (B200, when this came
+// in: 318.3 -> 276.3 and 202.4 -> 179.0 ms; now 264.4 and 140.8 ms).  The host
 // takes 20 to 50 us a pass to make a parameter block with or without it.
 // Per-instance tables and adjoint passes keep their matrices.
 #pragma nv_diag_suppress 20208  // long double: host code only here
@@ -356,13 +356,18 @@ struct Normaliser {
             state[size_t(o)] = 2;
             for (int e = 0; e < count(o); ++e) v[e] = mul(v[e], total);
             total = kOne;
-            begin = o + 1;
             taken = 0;
         };
         for (int o = 0; o < a.nops; ++o) {
             total = mul(total, late[size_t(o)]);
-            if (total.cl != 1 && free_diag(o)) put_back(o);
-            if (take_out(o) && ++taken == per_scalar) put_back(carrier(begin, o));
+            if (free_diag(o)) {
+                if (total.cl != 1) put_back(o);
+                begin = o;  // it can take the next ones as well, at no cost
+            }
+            if (take_out(o) && ++taken == per_scalar) {
+                put_back(carrier(begin, o));
+                begin = o + 1;
+            }
         }
         if (total.cl != 1) put_back(carrier(begin, a.nops - 1));
         double c = 0, h = 0, l = 0;
