@@ -57,7 +57,6 @@ def params(src, block):
 def _python(e):
     """A C expression of the generated text as a numpy expression."""
     e = re.sub(r"\b(\d+)u(?:ll)?\b", r"\1", e)
-    e = re.sub(r"\b(\d+)ull\b", r"\1", e)
     e = e.replace("u32(", "(").replace("&&", "&")
     return re.sub(r"p\.(\w+)\[", r"p['\1'][", e)
 
@@ -109,8 +108,7 @@ def run_launch(vec, src, block, norms=None):
             k, d, s = (int(x) for x in m.groups())
             dsm[d:d + k] = p["m"][s:s + k]
         elif m := re.match(r"const (?:u32|bool) (RD\d+|WR\d+|TH\d+|h\d+|c\d+) = (.*);", line):
-            if m.group(1) not in ("cur",):
-                env[m.group(1)] = eval(_python(m.group(2)), env)
+            env[m.group(1)] = eval(_python(m.group(2)), env)
         elif m := re.match(r"const V (v\d+) = (.*);", line):
             x = m.group(2)
             x = re.sub(r"make_(?:float|double)2\(0, 0\)", "zero", x)
